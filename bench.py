@@ -723,7 +723,7 @@ def run_ours(args, rank, world, local, pg):
             "plain": plain, "served": served, "roofline": roof, "cpu_baseline": cpu,
             "e2e": {"value": e2e, "unit": "queries/s", "h2d_bytes_per_step": h2d // args.steps,
                     "d2h_bytes_per_step": d2h // args.steps},
-            "schedule": [{"tile_variant": v, "driver": "graph" if dr else "host loop", "graph_error": ge}
+            "schedule": [{"tile_variant": v, "driver": ("host loop", "graph", "walk")[dr], "graph_error": ge}
                          for v, dr, ge in sorted(drivers)],
             "clocks": clk, "gpu_launches": launches, "ingest": ingest, "planner": planner, "ref_gpu": ref_gpu,
             "configs": configs,

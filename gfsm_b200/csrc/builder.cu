@@ -99,6 +99,31 @@ __global__ void k_symmetric(const unsigned long long *key, uint64_t m, uint32_t 
     }
 }
 
+// Row pointers by label group -- where each group's entries start in each row
+// (rows are id-sorted and a group is an id range) -- and the groups' entry
+// counts, a byte each.  starts: the groups' first ids.
+__global__ void k_row_groups(const uint32_t *rowptr, const uint32_t *adj, uint32_t n, uint32_t groups,
+                             const uint32_t *starts, uint32_t *rowgrp, unsigned long long *nlf) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const uint32_t re = rowptr[v + 1];
+        uint32_t p = rowptr[v];
+        unsigned long long have = 0;
+        for (uint32_t x = 0; x < groups; ++x) {
+            uint32_t lo = p, hi = re;  // the end of group x
+            while (lo < hi && x + 1 < groups) {
+                const uint32_t mid = lo + ((hi - lo) >> 1);
+                if (adj[mid] < starts[x + 1]) lo = mid + 1; else hi = mid;
+            }
+            const uint32_t e = x + 1 < groups ? lo : re;
+            if (groups > 1) rowgrp[(size_t)v * groups + x] = p;
+            have |= (unsigned long long)min(255u, e - p) << (8 * x);
+            p = e;
+        }
+        if (groups > 1 && v == n - 1) rowgrp[(size_t)n * groups] = re;
+        nlf[v] = have;
+    }
+}
+
 inline unsigned grid_for(uint64_t n, unsigned threads) {
     uint64_t b = (n + threads - 1) / threads;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(b, 148ull * 32));
@@ -109,8 +134,9 @@ inline unsigned grid_for(uint64_t n, unsigned threads) {
 void free_device_graph(DeviceGraph &g) {
     if (g.block) cudaFree(g.block);
     g.block = nullptr;
-    g.rowptr = g.adj = g.order = nullptr;
+    g.rowptr = g.adj = g.order = g.rowgrp = nullptr;
     g.elab = nullptr;
+    g.nlf = nullptr;
 }
 
 // Host side of the build.  The outputs (rowptr, adj, order, elab) live in one
@@ -147,6 +173,9 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     void *d_tmp;
     size_t tmp_bytes = 0, need = 0;
     int gbits = 0;
+    uint32_t groups = 1;
+    bool grouped = false;    // rows by label group (rowgrp, nlf)
+    uint64_t grp_words = 0;  // rowgrp's words, where it is not rowptr itself
     auto t_host0 = std::chrono::steady_clock::now();
 
     BCHECK(cudaSetDevice(device));
@@ -185,6 +214,9 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         out.group_start = {0, n};
     }
     while ((1ull << gbits) < out.group_value.size()) ++gbits;
+    groups = (uint32_t)out.group_value.size();
+    grouped = groups <= DeviceGraph::kMaxRowGroups && n;
+    if (grouped && groups > 1) grp_words = (uint64_t)n * groups + 1;
 
     // scratch sizes of the CUB passes (queried with null pointers)
     BCHECK(cub::DeviceRadixSort::SortPairs(nullptr, need, (unsigned long long *)nullptr,
@@ -202,12 +234,17 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     {
         // persistent outputs: rowptr | adj | order | elab
         const uint64_t o_rowptr = 0, o_adj = al((n1 + 1) * 4), o_order = o_adj + al(m1 * 4),
-                       o_elab = o_order + al(n1 * 4), o_end = o_elab + al(m1);
+                       o_elab = o_order + al(n1 * 4), o_grp = o_elab + al(m1), o_nlf = o_grp + al(grp_words * 4),
+                       o_end = o_nlf + (grouped ? al(n1 * 8) : 0);
         BCHECK(cudaMalloc(&out.block, o_end));
         char *b = static_cast<char *>(out.block);
         out.rowptr = reinterpret_cast<uint32_t *>(b + o_rowptr);
         out.adj = reinterpret_cast<uint32_t *>(b + o_adj);
         out.order = reinterpret_cast<uint32_t *>(b + o_order);
+        if (grouped) {
+            out.rowgrp = groups > 1 ? reinterpret_cast<uint32_t *>(b + o_grp) : out.rowptr;
+            out.nlf = reinterpret_cast<uint64_t *>(b + o_nlf);
+        }
         d_lab2 = reinterpret_cast<uint8_t *>(b + o_elab);  // becomes out.elab when labels differ
         // workspace
         const uint64_t sizes[] = {m1 * 4, m1 * 4, m1, n1 * 4, n1 * 4, n1 * 4, (n1 + 1) * 4, n1 * 4, 64,
@@ -285,6 +322,11 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         k_unpack<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.adj, d_lab2, d_flags);
         k_symmetric<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.rowptr, out.adj, d_flags);
     }
+    if (grouped) {
+        BCHECK(cudaMemcpyAsync(d_degs, out.group_start.data(), (uint64_t)groups * 4, cudaMemcpyHostToDevice, st));
+        k_row_groups<<<grid_for(n, 256), 256, 0, st>>>(out.rowptr, out.adj, n, groups, d_degs, out.rowgrp,
+                                                         reinterpret_cast<unsigned long long *>(out.nlf));
+    }
     BCHECK(cudaGetLastError());
     BCHECK(cudaEventRecord(ev[3], st));
     BCHECK(cudaMemcpyAsync(h_flags, d_flags, 12, cudaMemcpyDeviceToHost, st));
@@ -347,7 +389,8 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
             }
         }
     }
-    out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4;
+    out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4 + grp_words * 4 +
+                (grouped ? (uint64_t)n * 8 : 0);
     out.build_wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_host0).count();
 
 done:

@@ -43,6 +43,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "walk_launch.h"
 
 namespace gfsm {
 
@@ -1040,6 +1041,12 @@ const void *slot_kernel(int s, int ggeo, int kind) {
     return kind == 0 ? part[ggeo][s] : kind == 1 ? root[ggeo][s] : stepk[ggeo][s];
 }
 
+// Calls the walk takes (Engine::run): the longest data row, the least level
+// bounds (max_soln_size, max_scan_size) and the least arena.
+constexpr uint32_t kWalkMaxRow = 64;
+constexpr uint64_t kWalkMinLimit = 1ull << 20;
+constexpr uint64_t kWalkMinArena = 256ull << 20;
+
 inline uint64_t div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
 }  // namespace
@@ -1255,6 +1262,7 @@ gfsm_status Engine::init(int dev, uint64_t arena_limit, uint64_t scan_limit, std
         ECHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         ECHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm0, k_step_g<0, Geo0, false>, Geo0::T, 0));
         ECHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_step_g<0, Geo2, false>, Geo2::T, 0));
+        sm_count = sms;
         step_blocks[graph_geo(0)] = sms * std::max(per_sm0, 1);
         step_blocks[graph_geo(2)] = sms * std::max(per_sm2, 1);
     }
@@ -1270,6 +1278,19 @@ gfsm_status Engine::ensure_arena(uint64_t bytes, std::string &err) {
     arena_bytes = 0;
     ECHECK(cudaMalloc(&arena, bytes));
     arena_bytes = bytes;
+    return GFSM_OK;
+}
+
+gfsm_status Engine::ensure_stage(uint64_t bytes, std::string &err) {
+    if (h_stage_bytes >= bytes) return GFSM_OK;
+    // grown geometrically: freeing pinned memory synchronises the device,
+    // and served slots see batches of every size
+    const uint64_t want = std::max<uint64_t>({bytes, 2 * h_stage_bytes, 1ull << 20});
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = nullptr;
+    h_stage_bytes = 0;
+    ECHECK(cudaMallocHost(&h_stage, want));
+    h_stage_bytes = want;
     return GFSM_OK;
 }
 
@@ -1447,6 +1468,103 @@ int Engine::pick_variant(const std::vector<const Plan *> &plans, const DeviceGra
     return best;
 }
 
+// The walk over the active queries of a call.  ran = false: the tables do
+// not hold these plans (or the arena the tables), the level steps run.
+gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::vector<int> &active,
+                             const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
+                             const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
+                             const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran,
+                             std::string &err) {
+    ran = false;
+    const uint32_t na = (uint32_t)active.size();
+    const bool vl_on = lim.vertex_labels != 0;
+    std::vector<WalkQuery> ws(na);
+    for (uint32_t i = 0; i < na; ++i) {
+        const Plan *p = plans[active[i]];
+        ws[i] = {&dq[i], p, rlo[i], rhi[i], sym_ok && p->aut > 1 && p->sym_vl == vl_on};
+    }
+    const char *shr = getenv("GFSM_SHARE");
+    WalkTables &w = walk_tables;
+    struct Trim {
+        WalkTables &t;
+        ~Trim() { trim_walk(t); }
+    } trim{w};
+    // Symmetry conditions: any order of the data vertices keeps one embedding
+    // per orbit.  Ids ascend as degrees fall, so "the earlier vertex has the
+    // larger id" extends low-degree vertices by higher-degree ones and never
+    // enumerates a hub's row; a partitioned call keeps the ascending order,
+    // whose parts its callers have seen.
+    if (!build_walk(ws, g, na >= 2 && !(shr && *shr == '0'), !g.multi, true, nparts == 1, w)) return GFSM_OK;
+    auto al = [](uint64_t b) { return (b + 255) & ~255ull; };
+    const uint32_t nr = (uint32_t)w.root_lo.size();
+    const uint64_t o_counts = 256, o_nodes = o_counts + al(w.nslots * 8ull), o_sfx = o_nodes + al(w.nodes.size() * sizeof(WNode)),
+                   o_again = o_sfx + al(w.sfx.size() * sizeof(WSfx)),
+                   o_lo = o_again + al(w.again.size() * sizeof(WAgain)), o_off = o_lo + al(nr * 4ull),
+                   total = o_off + al((nr + 1) * 8ull);
+    // a call whose plans the level steps would refuse for MEMLIMIT stays theirs
+    const uint64_t level_head = 2ull * (na * (sizeof(DQuery) + 64ull) + (1ull << 20) * MAXQ);
+    const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count);
+    if (std::max(total + queue_bytes, level_head) > arena_cap / 2) return GFSM_OK;
+    ran = true;
+    gfsm_status rc = ensure_arena(arena_cap, err);
+    if (rc != GFSM_OK) return rc;
+    ECHECK(cudaStreamSynchronize(stream));  // a copy of an earlier call may still read the staging buffer
+    rc = ensure_stage(total, err);
+    if (rc != GFSM_OK) return rc;
+    char *hs = static_cast<char *>(h_stage), *ds = static_cast<char *>(arena);
+    std::memset(hs, 0, o_nodes);  // result and counts
+    std::memcpy(hs + o_nodes, w.nodes.data(), w.nodes.size() * sizeof(WNode));
+    if (!w.sfx.empty()) std::memcpy(hs + o_sfx, w.sfx.data(), w.sfx.size() * sizeof(WSfx));
+    if (!w.again.empty()) std::memcpy(hs + o_again, w.again.data(), w.again.size() * sizeof(WAgain));
+    std::memcpy(hs + o_lo, w.root_lo.data(), nr * 4ull);
+    std::memcpy(hs + o_off, w.root_off.data(), (nr + 1) * 8ull);
+    ECHECK(cudaMemcpyAsync(ds, hs, total, cudaMemcpyHostToDevice, stream));
+    WalkArgs a{};
+    // The neighbourhood filter is for batches (4,096 grid queries: 65.5 -> 56.4
+    // ms).  A lone query's walk is short (43 us with it, 51 without), and its
+    // peak_frontier_bytes, which the admission predictor is held against,
+    // stays that of the levels without the filter.
+    a.g = {g.rowptr, g.adj, g.elab, g.rowgrp, na > 1 ? g.nlf : nullptr, (uint32_t)g.group_value.size(), g.single_label, g.n, (uint32_t)g.m};
+    a.nodes = reinterpret_cast<const WNode *>(ds + o_nodes);
+    a.sfx = reinterpret_cast<const WSfx *>(ds + o_sfx);
+    a.again = reinterpret_cast<const WAgain *>(ds + o_again);
+    a.root_lo = reinterpret_cast<const uint32_t *>(ds + o_lo);
+    a.root_off = reinterpret_cast<const unsigned long long *>(ds + o_off);
+    a.roots = nr;
+    a.core = w.core;
+    a.node_count = (uint32_t)w.nodes.size();
+    a.sfxs = (uint32_t)w.sfx.size();
+    a.units = w.root_off[nr];
+    a.counts = reinterpret_cast<unsigned long long *>(ds + o_counts);
+    a.result = reinterpret_cast<WalkResult *>(ds);
+    a.queues = reinterpret_cast<Chunk *>(ds + total);
+    ECHECK(cudaEventRecord(ev0, stream));
+    ECHECK(launch_walk(a, g.elab || g.multi, sm_count, stream));
+    ECHECK(cudaEventRecord(ev1, stream));
+    const uint64_t back = o_counts + w.nslots * 8ull;
+    ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
+    ECHECK(cudaStreamSynchronize(stream));
+    const WalkResult *r = reinterpret_cast<const WalkResult *>(hs);
+    const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(hs + o_counts);
+    for (uint32_t i = 0; i < na; ++i) {
+        counts_out[active[i]] = cnt[w.slot[i]] * w.mult[i];
+        st.count += counts_out[active[i]];
+    }
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ev0, ev1);
+    st.kernel_ms = st.device_ms = ms;
+    st.steps = 1;
+    st.launches = 1;
+    st.candidates = r->candidates;
+    st.expansions = r->expansions;
+    st.alg_bytes = r->alg_bytes;
+    st.peak_frontier_bytes = std::min<uint64_t>(r->frontier_bytes, arena_cap);
+    st.h2d_bytes = total;
+    st.d2h_bytes = back;
+    st.driver = 2;
+    return GFSM_OK;
+}
+
 gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGraph &g, const gfsm_limits &lim,
                         uint64_t *counts_out, gfsm_stats *stats, uint32_t *rows_out, uint64_t max_rows,
                         uint64_t *n_rows, std::string &err, int variant, uint32_t part, uint32_t nparts) {
@@ -1470,7 +1588,20 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     const bool env_drv = drv && *drv;
     const bool force_graph = !trace && ((env_drv && !strcmp(drv, "graph")) || (!env_drv && tune_driver == 1));
     const bool force_host = trace || (env_drv && strcmp(drv, "graph")) || (!env_drv && tune_driver == 0);
-    if (variant < 0) variant = (plans.size() <= 1) ? 0 : pick_variant(plans, g, lim, err);
+    // The walk (walk.cu) takes counting calls on data of short rows: one lane
+    // per partial mapping is balanced there, and no level is written.  A call
+    // that names a level-step setting, caps its candidates or bounds its
+    // levels tightly gets the level steps, whose schedule those settings
+    // describe.
+    auto env_set = [](const char *n) {
+        const char *v = getenv(n);
+        return v && *v;
+    };
+    const bool walk = variant < 0 && !rows_out && !trace && g.max_degree <= kWalkMaxRow && !lim.max_candidates &&
+                      lim.max_soln_size >= kWalkMinLimit && lim.max_scan_size >= kWalkMinLimit &&
+                      arena_cap >= kWalkMinArena && tune_driver < 0 && !env_drv && !env_set("GFSM_TILE") &&
+                      !env_set("GFSM_SURVIVOR_GUESS");
+    if (variant < 0 && !walk) variant = (plans.size() <= 1) ? 0 : pick_variant(plans, g, lim, err);
     auto t_start = std::chrono::steady_clock::now();
     const int nq = (int)plans.size();
     gfsm_stats st{};
@@ -1479,7 +1610,9 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     ECHECK(cudaSetDevice(device));
 
     // device plans for the queries that can match at all
-    std::vector<DQuery> dq;
+    // (kept between walk calls: fresh pages cost as much as the plans)
+    std::vector<DQuery> own;
+    std::vector<DQuery> &dq = walk && nq <= (1 << 14) ? dq_kept : own;
     std::vector<int> active;
     std::vector<uint32_t> rlo, rhi;
     uint32_t dmax = 0;
@@ -1564,6 +1697,18 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     if (row_max * kWarpStage > 0xffffffffull) {
         err = "a data row of " + std::to_string(g.max_degree) + " entries exceeds the level step's 32-bit slice sums";
         return GFSM_ERR_TOO_LARGE;
+    }
+    if (walk) {
+        bool ran = false;
+        const gfsm_status rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, err);
+        if (ran) {
+            st.wall_ms =
+                std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
+            if (stats) *stats = st;
+            return rc;
+        }
+        return run(plans, g, lim, counts_out, stats, rows_out, max_rows, n_rows, err,
+                   plans.size() <= 1 ? 0 : pick_variant(plans, g, lim, err), part, nparts);
     }
     const uint64_t fan_cap = 0xffffffffull / (row_max * kWarpStage);
     std::vector<uint32_t> root_rep, fan_list, final_rep(na);
@@ -1695,16 +1840,8 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     // pinned staging buffer exactly as in the arena and sent with one copy.
     // A copy of an earlier call (one that returned early) may still read it.
     ECHECK(cudaStreamSynchronize(stream));
-    if (h_stage_bytes < head_used) {
-        // grown geometrically: freeing pinned memory synchronises the device,
-        // and served slots see batches of every size
-        const uint64_t want = std::max<uint64_t>({head_used, 2 * h_stage_bytes, 1ull << 20});
-        if (h_stage) cudaFreeHost(h_stage);
-        h_stage = nullptr;
-        h_stage_bytes = 0;
-        ECHECK(cudaMallocHost(&h_stage, want));
-        h_stage_bytes = want;
-    }
+    rc = ensure_stage(head_used, err);
+    if (rc != GFSM_OK) return rc;
     char *hs = static_cast<char *>(h_stage);
     auto host_of = [&](const void *dev) { return hs + (static_cast<const char *>(dev) - static_cast<char *>(arena)); };
     std::memcpy(host_of(d_plans), dq.data(), plans_bytes);

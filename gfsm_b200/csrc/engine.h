@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "gfsm_internal.h"
+#include "walk.h"
 
 namespace gfsm {
 
@@ -30,6 +31,9 @@ struct Engine {
     // graph-driven schedule (one graph launch per call; built once per engine)
     int arg_slot = -1;             // constant-memory slot for this engine's step arguments
     void *ctl = nullptr;           // device control block (inside the small region)
+    int sm_count = 0;
+    WalkTables walk_tables;        // the walk's tables and a call's device plans, reused by the next call
+    std::vector<DQuery> dq_kept;
     // one graph per tile geometry the schedule is instantiated for (two)
     int step_blocks[2] = {0, 0};   // fixed grid of the graph's step kernel
     cudaGraph_t graph[2] = {nullptr, nullptr};
@@ -44,6 +48,7 @@ struct Engine {
     void release();
     gfsm_status init(int dev, uint64_t arena_limit, uint64_t scan_limit, std::string &err);
     gfsm_status ensure_arena(uint64_t bytes, std::string &err);
+    gfsm_status ensure_stage(uint64_t bytes, std::string &err);
     // The graph-driven schedule for tile geometry `variant` (built once,
     // relaunched by every call); GFSM_ERR_CUDA where there is none.
     gfsm_status build_graph(int variant, std::string &err);
@@ -56,6 +61,10 @@ struct Engine {
     gfsm_status run(const std::vector<const Plan *> &plans, const DeviceGraph &g, const gfsm_limits &lim,
                     uint64_t *counts_out, gfsm_stats *stats, uint32_t *rows_out, uint64_t max_rows,
                     uint64_t *n_rows, std::string &err, int variant = -1, uint32_t part = 0, uint32_t nparts = 1);
+    gfsm_status run_walk(const std::vector<const Plan *> &plans, const std::vector<int> &active,
+                         const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
+                         const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
+                         const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, std::string &err);
     int pick_variant(const std::vector<const Plan *> &plans, const DeviceGraph &g, const gfsm_limits &lim,
                      std::string &err);
     std::map<uint64_t, int> tuned;  // autotuner: workload class -> tile geometry

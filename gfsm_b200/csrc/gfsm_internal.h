@@ -69,6 +69,11 @@ struct DeviceGraph {
     uint8_t *elab = nullptr;          // [m], null when every entry has the same label
     uint32_t single_label = 0;        // the label when elab == null
     uint32_t *order = nullptr;        // [n] internal id -> original id
+    // [n * groups + 1] row pointers by label group (WalkGraph::rowgrp); the
+    // row pointers themselves with one group, null with more than kMaxRowGroups
+    uint32_t *rowgrp = nullptr;
+    uint64_t *nlf = nullptr;          // [n] entries by label group, a byte each (WalkGraph::nlf); null with rowgrp
+    static constexpr uint32_t kMaxRowGroups = 8;
     void *block = nullptr;            // the one allocation rowptr, adj, order and elab live in
     bool symmetric = false, multi = false;
     int n_edge_labels = 0;

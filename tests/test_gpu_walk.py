@@ -1,0 +1,70 @@
+"""The walk (one kernel per call, data rows of at most 64 entries) against the
+level steps (GFSM_DRIVER=host) on the same device graph: every tuple length
+from 2 to 16 vertices, 1 to 300 queries a call (queues that fill and drain),
+more label groups than the row pointers by group hold, edge labels, repeated
+entries, a self-loop, and the longest row it takes and the next one."""
+import numpy as np
+import pytest
+
+import gfsm_b200
+from gfsm_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _counts(ctx, plans, data, monkeypatch, walked):
+    walk, st = ctx.batch_count(plans, data)
+    assert (st["driver"] == 2) == walked
+    monkeypatch.setenv("GFSM_DRIVER", "host")
+    level, st = ctx.batch_count(plans, data)
+    monkeypatch.delenv("GFSM_DRIVER")
+    assert st["driver"] == 0
+    assert walk.tolist() == level.tolist() and level.sum() > 0
+    # the parts of a partition as well
+    parts = [ctx.batch_count_part(plans, data, p, 3)[0] for p in range(3)]
+    assert sum(parts).tolist() == level.tolist()
+
+
+@pytest.mark.parametrize("nq", [1, 2, 33, 300])
+@pytest.mark.parametrize("form", ["labels", "nine_labels", "edge_labels", "repeated", "loop"])
+def test_walk_equals_level_steps(monkeypatch, form, nq):
+    ctx = gfsm_b200.GFSM(device=0, vertex_labels=1)
+    g = synth.grid(40, 0.05, 0.05, seed=nq)
+    g.vlabel = synth.vlabels(g.n, 9 if form == "nine_labels" else 3, 0.0, seed=4)
+    s, d = g.directed()
+    lab = np.ones(len(s), np.uint32)
+    if form == "edge_labels":
+        lab = 1 + (s ^ d) % 2
+    elif form == "repeated":
+        s, d, lab = np.append(s, s[:50]), np.append(d, d[:50]), np.append(lab, lab[:50])
+    elif form == "loop":
+        s, d, lab = np.append(s, [3, 9]), np.append(d, [3, 9]), np.append(lab, [1, 1])
+    data = ctx.graph_from_edges(g.n, s, d, lab, g.vlabel)
+    qs = []
+    for i in range(nq):
+        q, seen = synth.rw_query(g, 2 + i % 11 if nq > 1 else 7, tree=i % 2 == 0, seed=70 + i)
+        a, b = q.directed()
+        ql = 1 + (seen[a] ^ seen[b]) % 2 if form == "edge_labels" else np.ones(len(a), np.uint32)
+        qs.append((q.n, a, b, ql.astype(np.uint32), q.vlabel))
+    _counts(ctx, ctx.prepare_queries(qs), data, monkeypatch, True)
+    ctx.close()
+
+
+@pytest.mark.parametrize("row,walked", [(64, True), (65, False)])
+def test_longest_row(monkeypatch, row, walked):
+    """A star of `row` leaves beside a path and a cycle: long queries, 15
+    equal leaves (a falling factorial), leaves on several anchors."""
+    ctx = gfsm_b200.GFSM(device=0)
+    hub = [(0, i + 1) for i in range(row)]
+    n = row + 1
+    path = [(n + i, n + i + 1) for i in range(39)] + [(n + 39, n), (1, n), (2, n + 3)]
+    e = np.array(hub + path, np.uint32)
+    data = ctx.graph_from_edges(n + 40, np.concatenate([e[:, 0], e[:, 1]]), np.concatenate([e[:, 1], e[:, 0]]))
+    shapes = [[(i, i + 1) for i in range(15)], [(0, i + 1) for i in range(6)], [(0, 1), (1, 2), (0, 3), (0, 4), (2, 5)],
+              [(0, 1), (1, 2), (2, 3), (3, 0), (0, 4), (0, 5), (1, 6)], [(i, i + 1) for i in range(11)] + [(0, 12), (0, 13)]]
+    qs = []
+    for sh in shapes:
+        q = np.array(sh, np.uint32)
+        qs.append((int(q.max()) + 1, np.concatenate([q[:, 0], q[:, 1]]), np.concatenate([q[:, 1], q[:, 0]]), None, None))
+    _counts(ctx, ctx.prepare_queries(qs), data, monkeypatch, walked)
+    ctx.close()
