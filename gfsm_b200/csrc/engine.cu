@@ -135,7 +135,10 @@ struct StepArgs {
     const uint32_t *__restrict__ fan_list;
     // count a last query vertex when its parent is written, where nothing is
     // left to check (next_slice); only where the step's counts are committed
-    // after the step is accepted (a re-run step must not count twice)
+    // after the step is accepted (a re-run step must not count twice).
+    // 1: slices of short rows, and branching nodes whose children all end so;
+    // 2: every slice and every such child, and the next level's candidates
+    // come from the shortest row they must be in
     uint32_t leaf_count;
 };
 
@@ -144,7 +147,9 @@ struct StepArgs {
 // tuple's next-level slice (bit i = entry i) that are vertices of the tuple
 // itself -- they would fail injectivity, so they are not candidates.
 // kInjDone: that set is complete (the slice came from a short row), so the
-// next level need not compare its candidates with the tuple again.
+// next level need not compare its candidates with the tuple again.  Without
+// kInjDone, bits 22-29 name the row the slice came from: 0 the anchor's, r + 1
+// that of the next level's requirement r (whose place the anchor then takes).
 constexpr uint32_t kBranch = 1u << 31;
 constexpr uint32_t kInjDone = 1u << 30;
 constexpr uint32_t kExclShift = 22;
@@ -329,6 +334,21 @@ struct CandCtx {
     const uint32_t *rlo, *rhi, *rmode;
 };
 
+// How many vertices of the child's tuple (v and the parent's d) lie in the
+// slice adj[s, e) of the window [lo, hi).
+__device__ __forceinline__ uint32_t tuple_in_slice(const StepArgs &a, const uint32_t d, const uint32_t p, const uint32_t v,
+                                                   const uint32_t s, const uint32_t e, const uint32_t lo,
+                                                   const uint32_t hi) {
+    uint32_t n = 0;
+    for (uint32_t t = 0; t <= d; ++t) {
+        const uint32_t x = t == d ? v : __ldg(a.ptup + (uint64_t)(1 + t) * a.pstride + p);
+        if (x < lo || x >= hi) continue;
+        const uint32_t i = s + lower_bound_u32(a.g.adj + s, e - s, x);
+        n += i < e && __ldg(a.g.adj + i) == x;
+    }
+    return n;
+}
+
 // The child a surviving candidate becomes: its own candidate slice for
 // depth+1 (r.cs, r.cnt; r.q gains kBranch when its trie node branches).
 // False when the slice is empty -- such a child cannot be extended and is
@@ -385,46 +405,74 @@ __device__ __forceinline__ bool next_slice(const StepArgs &a, const uint32_t d, 
         if (khi < a.g.n) e = rs + lower_bound_u32(a.g.adj + rs, re - rs, khi);
     }
     if (e <= s) return false;
-    const uint32_t len = (e - s) - __popc(excl);
+    uint32_t len = (e - s) - __popc(excl);
     if (!len) return false;  // every entry of the slice is a vertex of the tuple
     // a branching node's child offers its slice to every child node
     const uint32_t nf = L->fan_count;
     const uint32_t mult = nf > 1 ? nf : 1u;
     // the child's tuple and anchor row, read once per (member) parent
     my_bytes += (4ull * (d + 1) + 4ull * (re - rs + 1)) * mult;
-    if (a.leaf_count && flags && !a.g.elab) {
-        // depth+1 is the last query vertex with nothing to check beyond the
-        // anchor edge (no requirement, no row search for the anchor): every
-        // entry left in the slice is an embedding -- count them here and
-        // write no child.  A branching node whose child nodes all end so
-        // (anchor_check bit 1) counts the slice once for each of them.
-        if (nf <= 1) {
+    uint32_t live = mult, qn = q;  // child nodes left to enumerate; the node the child is written under
+    if (a.leaf_count && !a.g.elab && (flags || a.leaf_count > 1)) {
+        // child nodes whose depth+1 is a last query vertex with nothing to
+        // check beyond the anchor edge (no requirement, no row search for the
+        // anchor): every entry of the slice outside the tuple is an embedding
+        // -- count them here and enumerate only the other child nodes.  A
+        // branching node lists those children last.  (64 three-vertex queries
+        // on a labelled R-MAT 2^20, nearly all paths: 2.41e9 -> 7.3e7
+        // candidates, 22.0 -> 2.7 ms.)
+        uint32_t leaves;
+        if (nf > 1) {
+            leaves = L->fan_leaves;
+            if (a.leaf_count == 1 && leaves < nf) leaves = 0;
+        } else {
             const DLevel *N = &a.plans[q].lv[d + 1];
-            if (N->final_ && N->nreq == 0 && !(N->anchor_check & 1u)) {
-                if (fc && q != fq) {
-                    atomicAdd(&a.counts[fq], fc);
-                    fc = 0;
-                }
-                fq = q;
-                fc += len;
-                return false;
-            }
-        } else if (L->anchor_check & 2u) {
-            for (uint32_t j = 0; j < nf; ++j) {
-                const uint32_t qj = __ldg(a.fan_list + L->fan_start + j);
+            leaves = N->final_ && N->nreq == 0 && !(N->anchor_check & 1u);
+        }
+        if (leaves) {
+            const uint32_t n = flags ? len : len - tuple_in_slice(a, d, p, v, s, e, klo, khi);
+            for (uint32_t j = 0; n && j < leaves; ++j) {
+                const uint32_t qj = nf > 1 ? __ldg(a.fan_list + L->fan_start + nf - leaves + j) : q;
                 if (fc && qj != fq) {
                     atomicAdd(&a.counts[fq], fc);
                     fc = 0;
                 }
                 fq = qj;
-                fc += len;
+                fc += n;
             }
-            return false;
+            live -= leaves;
+            if (!live) return false;
+            if (live == 1) qn = __ldg(a.fan_list + L->fan_start);
+        }
+    }
+    uint32_t mark = flags ? excl : 0u;
+    if (a.leaf_count > 1 && !flags && live == 1 && !a.g.elab) {
+        // A candidate of depth+1 must be in the anchor's row and in each
+        // requirement's: take it from the row with the fewest entries in the
+        // window, and check the anchor's instead.  On skewed graphs that is
+        // what bounds a triangle's wedges: R-MAT 2^20, 15.5M edges, 4.40e9
+        // candidates from the anchors' rows, 1.24e9 from the shortest (with
+        // orbits in descending id order), 71.8 -> 23.3 ms.
+        const DLevel *N = &a.plans[qn].lv[d + 1];
+        for (uint32_t t = 0; t < N->nreq && !(N->anchor_check & 1u); ++t) {
+            const uint32_t pos = N->req_pos[t];
+            if (pos == REQ_SELF) continue;
+            const uint32_t u = pos == d ? v : __ldg(a.ptup + (uint64_t)(1 + pos) * a.pstride + p);
+            const uint32_t us = __ldg(a.g.rowptr + u), ue = __ldg(a.g.rowptr + u + 1);
+            uint32_t s2 = us, e2 = ue;
+            if (klo) s2 = us + lower_bound_u32(a.g.adj + us, ue - us, klo);
+            if (khi < a.g.n) e2 = us + lower_bound_u32(a.g.adj + us, ue - us, khi);
+            if (e2 <= s2) return false;
+            if (e2 - s2 < len) {
+                s = s2;
+                len = e2 - s2;
+                mark = t + 1;
+            }
         }
     }
     r.cs = s;
-    r.cnt = len * mult;
-    r.q = q | (excl << kExclShift) | flags | (nf > 1 ? kBranch : 0u);
+    r.cnt = len * live;
+    r.q = qn | (mark << kExclShift) | flags | (live > 1 ? kBranch : 0u);
     return true;
 }
 
@@ -458,8 +506,9 @@ __device__ __forceinline__ void check_candidate(const StepArgs &a, const uint32_
     }
     const uint32_t p = t.plo + lo;
     uint32_t q = ROOT ? __ldg(a.root_rep + p) : __ldg(a.ptup + p);
-    const uint32_t excl = ROOT ? 0u : (q >> kExclShift) & 0xffu;
+    const uint32_t mark = ROOT ? 0u : (q >> kExclShift) & 0xffu;
     const bool inj_done = !ROOT && (q & kInjDone);
+    const uint32_t excl = inj_done ? mark : 0u, alt = inj_done ? 0u : mark;
     if (!ROOT && (q & kBranch)) {
         // the parent's trie node branches: its candidates run over (child
         // node, row offset), one copy of its slice per child node
@@ -474,7 +523,7 @@ __device__ __forceinline__ void check_candidate(const StepArgs &a, const uint32_
             span = local + (lo + 2 == t.nwin ? (uint32_t)(t.win_ends[1] - c) : (uint32_t)t.win[lo + 1] - off);
         else
             span = (uint32_t)(t.win[lo + 1] - t.win[lo]);
-        const uint32_t slen = span / P->fan_count;
+        const uint32_t slen = span / (P->fan_count - (a.leaf_count > 1 && !a.g.elab ? P->fan_leaves : 0u));
         const uint32_t j = local / slen;
         local -= j * slen;
         q = __ldg(a.fan_list + P->fan_start + j);
@@ -515,7 +564,7 @@ __device__ __forceinline__ void check_candidate(const StepArgs &a, const uint32_
     // remaining requirements (HnGPU.cu:243-252)
     for (uint32_t r = 0; r < L->nreq && (pass || acct); ++r) {
         const uint32_t mode = (t.single && r < (uint32_t)NSTAGE) ? t.rmode[r] : 0u;
-        const uint32_t pos = L->req_pos[r];
+        const uint32_t pos = r + 1 == alt ? L->anchor : L->req_pos[r];
         if (mode == 0u) {
             const uint32_t u = pos == REQ_SELF ? v : __ldg(a.ptup + (uint64_t)(1 + pos) * a.pstride + p);
             const uint32_t rs = __ldg(a.g.rowptr + u), re = __ldg(a.g.rowptr + u + 1);
@@ -594,11 +643,16 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, const uint32_t tile
 
     // ---- a tile inside one parent's slice (hub rows): stage the part of each
     // requirement row that can hold this tile's candidates
-    const bool single = !ROOT && plo == phi && a.g.elab == nullptr &&
-                        !(__ldg(a.ptup + plo) & (kBranch | (0xffu << kExclShift)));
+    bool single = !ROOT && plo == phi && a.g.elab == nullptr;
+    uint32_t qw = 0;  // the parent's column 0
     if (single) {
-        const uint32_t q0 = __ldg(a.ptup + plo) & kNodeMask;
-        const DLevel *L0 = &a.plans[q0].lv[d];
+        qw = __ldg(a.ptup + plo);
+        single = !(qw & kBranch) && (!(qw & kInjDone) || !(qw >> kExclShift & 0xffu));
+    }
+    if (single) {
+        const DLevel *L0 = &a.plans[qw & kNodeMask].lv[d];
+        const uint32_t alt = qw & kInjDone ? 0u : qw >> kExclShift & 0xffu;
+        auto req_pos = [&](uint32_t r) -> uint32_t { return r + 1 == alt ? L0->anchor : L0->req_pos[r]; };
         if (tid == 0) {
             const uint32_t cs0 = __ldg(a.pcstart + plo);
             const unsigned long long c00 = __ldg(a.pcoff + plo);
@@ -608,8 +662,8 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, const uint32_t tile
         __syncthreads();
         if (warp < 2 * NSTAGE) {
             const uint32_t r = warp >> 1;
-            if (r < L0->nreq && L0->req_pos[r] != REQ_SELF) {
-                const uint32_t u = __ldg(a.ptup + (uint64_t)(1 + L0->req_pos[r]) * a.pstride + plo);
+            if (r < L0->nreq && req_pos(r) != REQ_SELF) {
+                const uint32_t u = __ldg(a.ptup + (uint64_t)(1 + req_pos(r)) * a.pstride + plo);
                 const uint32_t rs = __ldg(a.g.rowptr + u), re = __ldg(a.g.rowptr + u + 1);
                 const uint32_t key = (warp & 1) ? sm.vlast + 1 : sm.vfirst;
                 const uint32_t b = rs + warp_lower_bound(a.g.adj + rs, re - rs, key, lane);
@@ -620,7 +674,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, const uint32_t tile
         }
         __syncthreads();
         for (uint32_t r = 0; r < (uint32_t)NSTAGE; ++r) {
-            if (r >= L0->nreq || L0->req_pos[r] == REQ_SELF) continue;
+            if (r >= L0->nreq || req_pos(r) == REQ_SELF) continue;
             const uint32_t lo = sm.rlo[r], n = sm.rhi[r] - sm.rlo[r];
             if (n <= (uint32_t)G::REQ)
                 for (uint32_t i = tid; i < n; i += T) sm.req[r][i] = __ldg(a.g.adj + lo + i);
@@ -1055,7 +1109,7 @@ inline uint64_t div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 // Device plan of one query against one data graph
 // ---------------------------------------------------------------------------
 gfsm_status build_dquery(const Plan &p, const DeviceGraph &g, const gfsm_limits &lim, DQuery &dq,
-                         uint32_t &root_lo, uint32_t &root_hi, bool &never, bool sym) {
+                         uint32_t &root_lo, uint32_t &root_hi, bool &never, bool sym, bool desc) {
     std::memset(&dq, 0, sizeof(dq));
     never = false;
     const uint32_t k = p.k;
@@ -1132,14 +1186,16 @@ gfsm_status build_dquery(const Plan &p, const DeviceGraph &g, const gfsm_limits 
         L.next_hi = N.hi;
     }
     if (sym) {
-        // f(a) < f(b): a bound on whichever of the two is placed later, taken
-        // from the earlier one's tuple position when its parent is written
+        // f(a) < f(b) (desc: >): a bound on whichever of the two is placed
+        // later, taken from the earlier one's tuple position when its parent
+        // is written
         std::vector<uint32_t> depth(k, 0);
         for (uint32_t d = 0; d < k; ++d) depth[p.qvid[d]] = d;
         for (const auto &c : p.sym_cond) {
             const uint32_t da = depth[c.first], db = depth[c.second];
-            if (da < db) dq.lv[db - 1].next_lb |= (uint16_t)(1u << da);
-            else dq.lv[da - 1].next_ub |= (uint16_t)(1u << db);
+            const uint32_t first = std::min(da, db), later = std::max(da, db);
+            DLevel &L = dq.lv[later - 1];
+            ((da < db) != desc ? L.next_lb : L.next_ub) |= (uint16_t)(1u << first);
         }
     }
     root_lo = lo[0];
@@ -1597,10 +1653,16 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         const char *v = getenv(n);
         return v && *v;
     };
-    const bool walk = variant < 0 && !rows_out && !trace && g.max_degree <= kWalkMaxRow && !lim.max_candidates &&
-                      lim.max_soln_size >= kWalkMinLimit && lim.max_scan_size >= kWalkMinLimit &&
-                      arena_cap >= kWalkMinArena && tune_driver < 0 && !env_drv && !env_set("GFSM_TILE") &&
-                      !env_set("GFSM_SURVIVOR_GUESS");
+    const bool roomy = !lim.max_candidates && lim.max_soln_size >= kWalkMinLimit &&
+                       lim.max_scan_size >= kWalkMinLimit && arena_cap >= kWalkMinArena;
+    const bool walk = variant < 0 && !rows_out && !trace && roomy && g.max_degree <= kWalkMaxRow && tune_driver < 0 &&
+                      !env_drv && !env_set("GFSM_TILE") && !env_set("GFSM_SURVIVOR_GUESS");
+    // The same calls' level steps count every last vertex they can at its
+    // parent, take candidates from the shortest row and, where symmetry is
+    // broken, order an orbit by descending id (low degrees first: see
+    // run_walk); others examine the candidates they always did, which a
+    // candidate cap counts and tight limits cut into steps.
+    const bool desc = roomy && nparts == 1;
     if (variant < 0 && !walk) variant = (plans.size() <= 1) ? 0 : pick_variant(plans, g, lim, err);
     auto t_start = std::chrono::steady_clock::now();
     const int nq = (int)plans.size();
@@ -1635,8 +1697,8 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         auto work = [&](int t) {
             for (int i = t; i < nq; i += nt) {
                 bool nv = false;
-                qrc[i] = build_dquery(*plans[i], g, lim, all[i], lo[i], hi[i], nv, sym_ok && plans[i]->aut > 1 &&
-                                                                                         plans[i]->sym_vl == vl_on);
+                qrc[i] = build_dquery(*plans[i], g, lim, all[i], lo[i], hi[i], nv,
+                                      sym_ok && plans[i]->aut > 1 && plans[i]->sym_vl == vl_on, desc);
                 never[i] = nv;
             }
         };
@@ -1777,13 +1839,18 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
                 if (kids.size() > 1) {
                     dq[r].lv[d].fan_count = (uint16_t)kids.size();
                     dq[r].lv[d].fan_start = (uint32_t)fan_list.size();
-                    bool leaves = true;  // every child node's depth d+1 is counted at its parent
-                    for (const auto &k : kids) {
-                        fan_list.push_back(k[0]);
+                    // children whose depth d+1 can be counted at the parent come last
+                    auto leaf = [&](const std::vector<uint32_t> &k) {
                         const DLevel &N = dq[k[0]].lv[d + 1];
-                        leaves = leaves && N.final_ && N.nreq == 0 && !(N.anchor_check & 1u);
-                    }
-                    if (leaves) dq[r].lv[d].anchor_check |= 2u;
+                        return N.final_ && N.nreq == 0 && !(N.anchor_check & 1u);
+                    };
+                    uint32_t leaves = 0;
+                    for (const auto &k : kids)
+                        if (leaf(k)) ++leaves;
+                        else fan_list.push_back(k[0]);
+                    for (const auto &k : kids)
+                        if (leaf(k)) fan_list.push_back(k[0]);
+                    dq[r].lv[d].fan_leaves = leaves;
                 }
                 // a node of one query has no fan-out below it and counts to
                 // itself: it is not carried to deeper levels
@@ -1794,7 +1861,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         }
         if (!share) {
             for (DQuery &q : dq)
-                for (DLevel &l : q.lv) l.fan_count = 0, l.fan_start = 0, l.anchor_check &= 1u;
+                for (DLevel &l : q.lv) l.fan_count = 0, l.fan_start = 0;
             fan_list.clear();
             root_rep.clear();
             for (uint32_t i = 0; i < na; ++i) final_rep[i] = i;
@@ -1977,7 +2044,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         a.rows_ctr = rows_ctr;
         a.root_rep = d_root_rep;
         a.fan_list = d_fan_list;
-        a.leaf_count = leaf_ok ? 1u : 0u;
+        a.leaf_count = leaf_ok ? (roomy ? 2u : 1u) : 0u;
         Ctl *d_ctl = static_cast<Ctl *>(ctl);
         ECHECK(cudaMemcpyAsync(d_ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, stream));
         st.h2d_bytes += sizeof(Ctl);
@@ -2086,7 +2153,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         a.rows_ctr = rows_ctr;
         a.root_rep = d_root_rep;
         a.fan_list = d_fan_list;
-        a.leaf_count = leaf_ok ? 1u : 0u;
+        a.leaf_count = leaf_ok ? (roomy ? 2u : 1u) : 0u;
         a.pcoff_end = total[d];
         k_partition<<<(unsigned)div_up((uint64_t)std::max<uint32_t>(ntiles + 1, ne), 256), 256, 0, stream>>>(
             a.pcoff, a.np, a.pcoff_end, a.c0, chunk, ntiles, vtile, tile_parent, d_result, d_step_counts, ne);

@@ -123,16 +123,20 @@ struct Plan {
 
 // Per-depth device plan of one query against one data graph.
 struct alignas(16) DLevel {
-    uint32_t lo, hi;           // candidate id window of this depth
+    union {
+        uint32_t lo;           // candidate id window of this depth: its start (host) ...
+        uint32_t fan_leaves;   // ... in a branching trie node's representative, once the trie is built:
+                               // how many of its child nodes, the last ones in fan_list, are a last
+                               // vertex that is counted at its parent
+    };
+    uint32_t hi;               // end of the window
     uint32_t next_lo, next_hi; // window of depth+1
     uint8_t anchor;            // tuple position of the anchor (depth index)
     uint8_t next_anchor;       // anchor position for depth+1
     uint8_t nreq;              // extra requirement checks
     uint8_t anchor_lab;        // label of the anchor requirement
     uint8_t final_;            // depth == k-1
-    uint8_t anchor_check;      // bit 0: the anchor requirement needs a row search (multi-edge
-                               // data); bit 1 (a branching trie node's representative): every
-                               // child node's depth+1 is a last vertex counted at its parent
+    uint8_t anchor_check;      // bit 0: the anchor requirement needs a row search (multi-edge data)
     uint16_t next_ub;          // symmetry breaking: depth+1's candidate < tuple[pos] for these positions
     uint8_t req_pos[MAXQ];     // tuple position, or REQ_SELF
     uint8_t req_lab[MAXQ];
@@ -259,9 +263,10 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
 void free_device_graph(DeviceGraph &g);
 // engine.cu
 // sym: also encode the plan's symmetry-breaking conditions (the caller then
-// multiplies the count by p.aut).
+// multiplies the count by p.aut); desc: reversed, f(a) > f(b).
 gfsm_status build_dquery(const Plan &p, const DeviceGraph &g, const gfsm_limits &lim,
-                         DQuery &dq, uint32_t &root_lo, uint32_t &root_hi, bool &never, bool sym = false);
+                         DQuery &dq, uint32_t &root_lo, uint32_t &root_hi, bool &never, bool sym = false,
+                         bool desc = false);
 // Device bytes one partial mapping of depth d's buffer takes: query id and
 // d+1 tuple columns, its next-level slice start and candidate prefix.
 #ifdef __CUDACC__
