@@ -1098,6 +1098,9 @@ const void *slot_kernel(int s, int ggeo, int kind) {
 // Calls the walk takes (Engine::run): the longest data row, the least level
 // bounds (max_soln_size, max_scan_size) and the least arena.
 constexpr uint32_t kWalkMaxRow = 64;
+// Longer rows: the longest row's share of one label group, for which a light
+// call tries the walk (kWalkRounds rounds a warp at most, 1 to 2 us each).
+constexpr uint32_t kWalkMaxGroupRow = 1024;
 constexpr uint64_t kWalkMinLimit = 1ull << 20;
 constexpr uint64_t kWalkMinArena = 256ull << 20;
 
@@ -1529,7 +1532,7 @@ int Engine::pick_variant(const std::vector<const Plan *> &plans, const DeviceGra
 gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::vector<int> &active,
                              const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
                              const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
-                             const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran,
+                             const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, bool limited,
                              std::string &err) {
     ran = false;
     const uint32_t na = (uint32_t)active.size();
@@ -1550,17 +1553,22 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     // larger id" extends low-degree vertices by higher-degree ones and never
     // enumerates a hub's row; a partitioned call keeps the ascending order,
     // whose parts its callers have seen.
-    if (!build_walk(ws, g, na >= 2 && !(shr && *shr == '0'), !g.multi, true, nparts == 1, w)) return GFSM_OK;
+    if (!build_walk(ws, g, na >= 2 && !(shr && *shr == '0'), !g.multi, !limited, nparts == 1, w)) return GFSM_OK;
     auto al = [](uint64_t b) { return (b + 255) & ~255ull; };
+    // an entry's candidates (a row's slice for each child node) stay below
+    // 2^22, so that the walk's quotients and sums over a queue are exact
+    uint32_t kids = 1;
+    for (const WNode &n : w.nodes) kids = std::max<uint32_t>(kids, n.nchild);
+    if ((uint64_t)kids * g.max_degree >= (1ull << 22)) return GFSM_OK;
     const uint32_t nr = (uint32_t)w.root_lo.size();
-    const uint64_t o_counts = 256, o_nodes = o_counts + al(w.nslots * 8ull), o_sfx = o_nodes + al(w.nodes.size() * sizeof(WNode)),
+    const uint64_t o_counts = al(sizeof(WalkResult)), o_nodes = o_counts + al(w.nslots * 8ull), o_sfx = o_nodes + al(w.nodes.size() * sizeof(WNode)),
                    o_again = o_sfx + al(w.sfx.size() * sizeof(WSfx)),
                    o_lo = o_again + al(w.again.size() * sizeof(WAgain)), o_off = o_lo + al(nr * 4ull),
                    total = o_off + al((nr + 1) * 8ull);
     // a call whose plans the level steps would refuse for MEMLIMIT stays theirs
     const uint64_t level_head = 2ull * (na * (sizeof(DQuery) + 64ull) + (1ull << 20) * MAXQ);
-    const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count);
-    if (std::max(total + queue_bytes, level_head) > arena_cap / 2) return GFSM_OK;
+    const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count), list_bytes = limited ? walk_list_bytes(w.core) : 0;
+    if (std::max(total + queue_bytes + list_bytes, level_head) > arena_cap / 2) return GFSM_OK;
     ran = true;
     gfsm_status rc = ensure_arena(arena_cap, err);
     if (rc != GFSM_OK) return rc;
@@ -1595,12 +1603,18 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     a.result = reinterpret_cast<WalkResult *>(ds);
     a.queues = reinterpret_cast<Chunk *>(ds + total);
     ECHECK(cudaEventRecord(ev0, stream));
-    ECHECK(launch_walk(a, g.elab || g.multi, sm_count, stream));
+    ECHECK(launch_walk(a, g.elab || g.multi, limited, reinterpret_cast<Chunk *>(ds + total + queue_bytes), sm_count, stream));
     ECHECK(cudaEventRecord(ev1, stream));
     const uint64_t back = o_counts + w.nslots * 8ull;
     ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
     ECHECK(cudaStreamSynchronize(stream));
     const WalkResult *r = reinterpret_cast<const WalkResult *>(hs);
+    bool rest = r->gave_up != 0 || r->unit < a.units;  // work that no pass took on
+    for (int p = 0; limited && p + 1 < kWalkPasses; ++p) rest = rest || r->taken[p] < std::min(r->listed[p], kWalkListed);
+    if (rest) {
+        ran = false;
+        return GFSM_OK;
+    }
     const unsigned long long *cnt = reinterpret_cast<const unsigned long long *>(hs + o_counts);
     for (uint32_t i = 0; i < na; ++i) {
         counts_out[active[i]] = cnt[w.slot[i]] * w.mult[i];
@@ -1609,12 +1623,14 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     st.kernel_ms = st.device_ms = ms;
-    st.steps = 1;
-    st.launches = 1;
-    st.candidates = r->candidates;
-    st.expansions = r->expansions;
-    st.alg_bytes = r->alg_bytes;
-    st.peak_frontier_bytes = std::min<uint64_t>(r->frontier_bytes, arena_cap);
+    st.steps = st.launches = limited ? kWalkPasses : 1;
+    for (const auto &t : r->total) {
+        st.candidates += t[0];
+        st.expansions += t[1];
+        st.alg_bytes += t[2];
+        st.peak_frontier_bytes += t[3];
+    }
+    st.peak_frontier_bytes = std::min<uint64_t>(st.peak_frontier_bytes, arena_cap);
     st.h2d_bytes = total;
     st.d2h_bytes = back;
     st.driver = 2;
@@ -1655,8 +1671,12 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     };
     const bool roomy = !lim.max_candidates && lim.max_soln_size >= kWalkMinLimit &&
                        lim.max_scan_size >= kWalkMinLimit && arena_cap >= kWalkMinArena;
-    const bool walk = variant < 0 && !rows_out && !trace && roomy && g.max_degree <= kWalkMaxRow && tune_driver < 0 &&
-                      !env_drv && !env_set("GFSM_TILE") && !env_set("GFSM_SURVIVOR_GUESS");
+    // Data with longer rows whose label groups still are short has the walk
+    // try light calls (below).
+    const bool short_rows = g.max_degree <= kWalkMaxRow;
+    const bool walk = variant < 0 && !rows_out && !trace && roomy && tune_driver < 0 && !env_drv &&
+                      !env_set("GFSM_TILE") && !env_set("GFSM_SURVIVOR_GUESS") &&
+                      (short_rows || g.max_degree <= kWalkMaxGroupRow * g.group_value.size());
     // The same calls' level steps count every last vertex they can at its
     // parent, take candidates from the shortest row and, where symmetry is
     // broken, order an orbit by descending id (low degrees first: see
@@ -1762,8 +1782,29 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     }
     if (walk) {
         bool ran = false;
-        const gfsm_status rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, err);
-        if (ran) {
+        gfsm_status rc = GFSM_OK;
+        if (short_rows) {
+            rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, false, err);
+        } else {
+            uint64_t entries = 0;
+            for (uint32_t i = 0; i < na && entries <= kGraphRootEntries; ++i)
+                entries += (uint64_t)g.h_rowptr[rhi[i]] - g.h_rowptr[rlo[i]];
+            if (entries <= kGraphRootEntries) {
+                Skip &skip = walk_skip[workload_class(plans, g)];
+                if (skip.left) {
+                    --skip.left;
+                } else {
+                    rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, true, err);
+                    if (ran) {
+                        skip.next = 8;
+                    } else if (rc == GFSM_OK) {
+                        skip.left = skip.next;
+                        skip.next = std::min(2 * skip.next, 4096u);
+                    }
+                }
+            }
+        }
+        if (ran || rc != GFSM_OK) {
             st.wall_ms =
                 std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
             if (stats) *stats = st;

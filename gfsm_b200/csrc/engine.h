@@ -34,6 +34,12 @@ struct Engine {
     int sm_count = 0;
     WalkTables walk_tables;        // the walk's tables and a call's device plans, reused by the next call
     std::vector<DQuery> dq_kept;
+    // walks on long-row data that gave up, per workload class: how many calls
+    // to leave to the level steps before the next try, and how many after that
+    struct Skip {
+        uint32_t left = 0, next = 8;
+    };
+    std::map<uint64_t, Skip> walk_skip;
     // one graph per tile geometry the schedule is instantiated for (two)
     int step_blocks[2] = {0, 0};   // fixed grid of the graph's step kernel
     cudaGraph_t graph[2] = {nullptr, nullptr};
@@ -64,7 +70,8 @@ struct Engine {
     gfsm_status run_walk(const std::vector<const Plan *> &plans, const std::vector<int> &active,
                          const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
                          const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
-                         const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, std::string &err);
+                         const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, bool limited,
+                         std::string &err);
     int pick_variant(const std::vector<const Plan *> &plans, const DeviceGraph &g, const gfsm_limits &lim,
                      std::string &err);
     std::map<uint64_t, int> tuned;  // autotuner: workload class -> tile geometry

@@ -86,9 +86,12 @@ __device__ __forceinline__ void deal(uint32_t n, uint32_t lane, uint32_t &incl, 
     local = lane - __shfl_sync(kFull, excl, from);
 }
 
-template <bool LAB>
+// LIM: a pass of a limited walk (as a run-time switch its code cost the
+// unlimited walk 12%).
+template <bool LAB, bool LIM>
 __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) {
     extern __shared__ __align__(16) uint32_t sh[];
+    __shared__ unsigned long long cta_sum[kWarps][4];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
     const Tuple t{sh + (warp * tuple_chunks(a.core) * 32 + lane) * 4, 128};  // this lane's candidate's tuple
     Chunk *const queues = a.queues + (size_t)(blockIdx.x * kWarps + warp) * a.warp_chunks;
@@ -100,6 +103,42 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
     unsigned long long fcount = 0;
     unsigned long long u_next = 0, u_end = 0;  // this warp's units
     bool more = true;
+    uint32_t rounds = 0;
+    // units of the list (l_end == 0: none left), dealt a few at a time
+    const uint32_t l_count = LIM && a.pass ? min(__ldcg(&a.result->listed[a.pass - 1]), kWalkListed) : 0u;
+    const uint32_t l_chunk = max(1u, min(32u, l_count / (gridDim.x * kWarps)));
+    uint32_t l_next = 1, l_end = l_count ? 1u : 0u;
+    const uint32_t unit_chunks = 1 + tuple_chunks(a.core) + 1;
+    // n units, a lane each, into the queues of their depths
+    auto take_units = [&](uint32_t first, uint32_t n) {
+        const Chunk *const u = a.list_in + (size_t)(first + lane) * unit_chunks;
+        const bool has = lane < n;
+        Chunk h{0, 0, 0, 0};
+        uint32_t d = 0;
+        if (has) {
+            h = u[0];
+            d = u[1].x;
+        }
+        for (uint32_t rest = __ballot_sync(kFull, has); rest;) {
+            const uint32_t depth = __shfl_sync(kFull, d, __ffs(rest) - 1);
+            const uint32_t same = __ballot_sync(kFull, has && d == depth);
+            const uint32_t e0 = __shfl_sync(kFull, ents, depth);
+            Chunk *const q = queues + __shfl_sync(kFull, base, depth);
+            const bool mine = has && d == depth;
+            if (mine) {
+                const uint32_t e = (e0 + __popc(same & below)) % kQueue;
+                q[e] = h;
+                for (uint32_t x = 0; x * 4 < depth; ++x) q[(1 + x) * kQueue + e] = u[2 + x];
+            }
+            const uint32_t got = __reduce_add_sync(kFull, mine ? h.w : 0u);
+            if (lane == depth) {
+                ents = e0 + __popc(same);
+                left += got;
+            }
+            rest &= ~same;
+        }
+        __syncwarp();
+    };
     auto add = [&](uint32_t slot, unsigned long long n) {
         if (fslot != slot && fcount) {
             atomicAdd(a.counts + fslot, fcount);
@@ -115,13 +154,41 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         const uint32_t full = __ballot_sync(kFull, left >= 32), any = __ballot_sync(kFull, left != 0);
         uint32_t d = 0;
         bool sfx = spairs >= 32;
+        const bool closing = LIM && ++rounds > a.max_rounds;
+        if (closing && !sfx) {
+            if (!spairs) break;
+            sfx = true;
+        }
         if (!sfx) {
             if (full) {
                 d = 31 - __clz(full);
             } else {
+                if (LIM && l_end) {  // units that the pass before left come first
+                    if (l_next >= l_end) {
+                        uint32_t u = 0;
+                        if (lane == 0) {
+                            u = __ldcg(&a.result->taken[a.pass - 1]);
+                            if (u < l_count) u = atomicAdd(&a.result->taken[a.pass - 1], l_chunk);
+                        }
+                        l_next = __shfl_sync(kFull, u, 0);
+                        l_end = min(l_next + l_chunk, l_count);
+                        if (l_next >= l_count) l_next = l_end = 0;
+                    }
+                    if (l_end) {
+                        take_units(l_next, min(l_end - l_next, 32u));
+                        l_next += 32;
+                        continue;
+                    }
+                }
                 if (more && u_next >= u_end) {
+                    // (a warp's first take goes straight to the counter; later it
+                    // looks whether any are left: 5,920 warps adding to one
+                    // word just to find out took 20 us)
                     unsigned long long u = 0;
-                    if (lane == 0) u = atomicAdd(&a.result->unit, (unsigned long long)a.chunk);
+                    if (lane == 0) {
+                        if (u_end || (LIM && a.pass)) u = __ldcg(&a.result->unit);
+                        if (u < a.units) u = atomicAdd(&a.result->unit, (unsigned long long)a.chunk);
+                    }
                     u_next = __shfl_sync(kFull, u, 0);
                     u_end = min(u_next + a.chunk, a.units);
                     more = u_next < a.units;
@@ -166,7 +233,9 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                     uint32_t first = 0;
                     const unsigned long long ways = suffix_count<LAB>(a.g, sx, t, nc, bytes, first);
                     if (ways) add(__ldg(&sx->slot), ways);
-                    if (__ldg(&sx->nleaf) > 1 && first) front += (uint32_t)tuple_bytes(nc - 1);
+                    const uint32_t nleaf = __ldg(&sx->nleaf);
+                    if (nleaf > 1 && first) front += (uint32_t)tuple_bytes(nc - 1);
+                    if (nleaf > 2) front += first * (uint32_t)tuple_bytes(nc);
                 }
                 __syncwarp();
                 continue;
@@ -250,14 +319,60 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         }
         __syncwarp();  // queue entries are read by other lanes next
     }
-    if (fcount) atomicAdd(a.counts + fslot, fcount);
-    const unsigned long long c64 = warp_total(cand), k64 = warp_total(kept), b64 = warp_total(bytes),
-                             f64 = warp_total(front);
-    if (lane == 0) {
-        atomicAdd(&a.result->candidates, c64);
-        atomicAdd(&a.result->expansions, k64);
-        atomicAdd(&a.result->alg_bytes, b64);
-        atomicAdd(&a.result->frontier_bytes, f64);
+    // ---- what a limited pass leaves: every queue entry as units of about 32
+    // candidates (at most 64 to an entry), whole children or parts of one slice
+    if (LIM && __any_sync(kFull, left != 0)) {
+        if (!a.list_out) {
+            if (lane == 0) a.result->gave_up = 1;
+        } else {
+            for (uint32_t d = 1; d < a.core; ++d) {
+                const Chunk *const q = queues + __shfl_sync(kFull, base, d);
+                const uint32_t n = min(__shfl_sync(kFull, ents, d), kQueue);
+                for (uint32_t e = lane; e < n; e += 32) {
+                    const Chunk h = q[e];
+                    const uint32_t size = max(32u, (h.w + 63) / 64);
+                    // children whole in groups (short slices), else one by one in parts
+                    const uint32_t group = max(1u, size / max(h.z, 1u));
+                    for (uint32_t at = 0; at < h.w;) {
+                        const uint32_t j = at / h.z, i = at - j * h.z;
+                        Chunk u{h.x + j, h.y + i, min(min(h.z - i, size), h.w - at), 0};
+                        u.w = u.z;
+                        if (i == 0 && u.z == h.z) u.w = h.z * min(group, (h.w - at) / h.z);
+                        at += u.w;
+                        const uint32_t slot = atomicAdd(&a.result->listed[a.pass], 1u);
+                        if (slot >= kWalkListed) {
+                            a.result->gave_up = 1;
+                            break;
+                        }
+                        Chunk *const o = a.list_out + (size_t)slot * unit_chunks;
+                        o[0] = u;
+                        o[1] = Chunk{d, 0, 0, 0};
+                        for (uint32_t x = 0; x * 4 < d; ++x) o[2 + x] = q[(1 + x) * kQueue + e];
+                    }
+                }
+            }
+        }
+    }
+    // ---- counts and totals.  5,920 warps adding to the same words one by one
+    // took 25 us: a warp whose lanes hold one slot's count adds once, a CTA its
+    // totals once, to one of kWalkTotals places.
+    const uint32_t hold = __ballot_sync(kFull, fcount != 0);
+    if (hold) {
+        const uint32_t slot = __shfl_sync(kFull, fslot, __ffs(hold) - 1);
+        if (__all_sync(kFull, fcount == 0 || fslot == slot)) {
+            const unsigned long long n = warp_total(fcount);
+            if (lane == 0) atomicAdd(a.counts + slot, n);
+        } else if (fcount) {
+            atomicAdd(a.counts + fslot, fcount);
+        }
+    }
+    const unsigned long long sum[4] = {warp_total(cand), warp_total(kept), warp_total(bytes), warp_total(front)};
+    if (lane < 4) cta_sum[warp][lane] = lane < 2 ? (lane ? sum[1] : sum[0]) : (lane == 3 ? sum[3] : sum[2]);
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        unsigned long long n = 0;
+        for (uint32_t w = 0; w < kWarps; ++w) n += cta_sum[w][threadIdx.x];
+        if (n) atomicAdd(&a.result->total[blockIdx.x % kWalkTotals][threadIdx.x], n);
     }
 }
 
@@ -267,7 +382,9 @@ uint64_t walk_queue_bytes(uint32_t core, int sms) {
     return (uint64_t)sms * kCtas * kWarps * queue_chunks(core) * 16;
 }
 
-cudaError_t launch_walk(const WalkArgs &args, bool lab, int sms, cudaStream_t st) {
+uint64_t walk_list_bytes(uint32_t core) { return 2ull * kWalkListed * (2 + tuple_chunks(core)) * 16; }
+
+cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int sms, cudaStream_t st) {
     WalkArgs a = args;
     const uint32_t smem = tuple_chunks(a.core) * 32 * 16 * kWarps;
     a.warp_chunks = queue_chunks(a.core);
@@ -276,14 +393,24 @@ cudaError_t launch_walk(const WalkArgs &args, bool lab, int sms, cudaStream_t st
     // than 32 where there is not enough for all of them, so that a small
     // call's roots spread over the whole chip.
     unsigned long long chunk = a.units / (warps * 16) / 32 * 32;
-    chunk = std::min<unsigned long long>(256, std::max<unsigned long long>(chunk, 32));
+    chunk = std::min<unsigned long long>(limited ? 32 : 256, std::max<unsigned long long>(chunk, 32));
     if (a.units < warps * 32) chunk = std::max<unsigned long long>(1, (a.units + warps - 1) / warps);
     a.chunk = (uint32_t)chunk;
     const unsigned long long need = (a.units + chunk - 1) / chunk;
-    const uint32_t ctas = (uint32_t)std::max<unsigned long long>(
-        1, std::min<unsigned long long>((unsigned long long)sms * kCtas, (need + kWarps - 1) / kWarps));
-    if (lab) k_walk<true><<<ctas, kWalkThreads, smem, st>>>(a);
-    else k_walk<false><<<ctas, kWalkThreads, smem, st>>>(a);
+    const uint32_t all = (uint32_t)sms * kCtas;
+    const uint32_t first = (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(all, (need + kWarps - 1) / kWarps));
+    Chunk *const list[2] = {lists, lists + (size_t)kWalkListed * (2 + tuple_chunks(a.core))};
+    for (int p = 0; p < (limited ? kWalkPasses : 1); ++p) {
+        a.pass = (uint32_t)p;
+        a.max_rounds = limited ? kWalkRounds[p] : 0;
+        a.list_in = p ? list[(p - 1) & 1] : nullptr;
+        a.list_out = limited && p + 1 < kWalkPasses ? list[p & 1] : nullptr;
+        const uint32_t ctas = p ? all : first;
+        if (lab && limited) k_walk<true, true><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (lab) k_walk<true, false><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (limited) k_walk<false, true><<<ctas, kWalkThreads, smem, st>>>(a);
+        else k_walk<false, false><<<ctas, kWalkThreads, smem, st>>>(a);
+    }
     return cudaGetLastError();
 }
 

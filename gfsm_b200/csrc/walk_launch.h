@@ -9,11 +9,23 @@
 namespace gfsm {
 
 constexpr int kWalkThreads = 128;
+// A limited walk (Engine::run_walk) is a few passes: a warp that has taken a
+// pass's rounds writes what is left in its queues to a list, and the next
+// pass deals the list to all warps.  What the last one leaves is not walked.
+constexpr int kWalkPasses = 3;
+constexpr uint32_t kWalkRounds[kWalkPasses] = {24, 48, 192};
+constexpr uint32_t kWalkListed = 1u << 18;  // units a list holds
+
+constexpr int kWalkTotals = 32;
 
 struct WalkResult {
     unsigned long long unit;  // units handed out so far
-    unsigned long long candidates, expansions, alg_bytes;
-    unsigned long long frontier_bytes;  // of the partial mappings extended: what whole levels would hold
+    uint32_t gave_up;  // the last pass left work: the counts are not complete
+    uint32_t listed[kWalkPasses];  // work units each pass left to the next ...
+    uint32_t taken[kWalkPasses];   // ... and how many of them that one has handed out
+    // candidates, expansions, algorithmic bytes and the bytes of the partial
+    // mappings extended (what whole levels would hold), in parts
+    unsigned long long total[kWalkTotals][4];
 };
 
 struct WalkArgs {
@@ -28,11 +40,19 @@ struct WalkArgs {
     unsigned long long *counts;  // per slot
     WalkResult *result;
     Chunk *queues;            // walk_queue_bytes(core, sms) of scratch
+    // limited walks only: this pass, its rounds, what the one before left,
+    // where it leaves its own
+    uint32_t pass, max_rounds;
+    const Chunk *list_in;
+    Chunk *list_out;
     uint32_t chunk, warp_chunks;  // set by launch_walk
 };
 
 // Bytes of the warps' queues for tuples of up to `core` vertices.
 uint64_t walk_queue_bytes(uint32_t core, int sms);
-cudaError_t launch_walk(const WalkArgs &args, bool lab, int sms, cudaStream_t st);
+// Bytes of the two lists of a limited walk.
+uint64_t walk_list_bytes(uint32_t core);
+// limited: kWalkPasses passes, with `lists` for what they leave one another.
+cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int sms, cudaStream_t st);
 
 }  // namespace gfsm
