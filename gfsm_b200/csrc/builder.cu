@@ -116,11 +116,11 @@ __global__ void k_row_groups(const uint32_t *rowptr, const uint32_t *adj, uint32
             }
             const uint32_t e = x + 1 < groups ? lo : re;
             if (groups > 1) rowgrp[(size_t)v * groups + x] = p;
-            have |= (unsigned long long)min(255u, e - p) << (8 * x);
+            if (nlf) have |= (unsigned long long)min(255u, e - p) << (8 * x);
             p = e;
         }
         if (groups > 1 && v == n - 1) rowgrp[(size_t)n * groups] = re;
-        nlf[v] = have;
+        if (nlf) nlf[v] = have;
     }
 }
 
@@ -235,7 +235,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         // persistent outputs: rowptr | adj | order | elab
         const uint64_t o_rowptr = 0, o_adj = al((n1 + 1) * 4), o_order = o_adj + al(m1 * 4),
                        o_elab = o_order + al(n1 * 4), o_grp = o_elab + al(m1), o_nlf = o_grp + al(grp_words * 4),
-                       o_end = o_nlf + (grouped ? al(n1 * 8) : 0);
+                       o_end = o_nlf + (groups <= 8 ? al(n1 * 8) : 0);
         BCHECK(cudaMalloc(&out.block, o_end));
         char *b = static_cast<char *>(out.block);
         out.rowptr = reinterpret_cast<uint32_t *>(b + o_rowptr);
@@ -243,7 +243,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         out.order = reinterpret_cast<uint32_t *>(b + o_order);
         if (grouped) {
             out.rowgrp = groups > 1 ? reinterpret_cast<uint32_t *>(b + o_grp) : out.rowptr;
-            out.nlf = reinterpret_cast<uint64_t *>(b + o_nlf);
+            if (groups <= 8) out.nlf = reinterpret_cast<uint64_t *>(b + o_nlf);
         }
         d_lab2 = reinterpret_cast<uint8_t *>(b + o_elab);  // becomes out.elab when labels differ
         // workspace
@@ -390,7 +390,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         }
     }
     out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4 + grp_words * 4 +
-                (grouped ? (uint64_t)n * 8 : 0);
+                (out.nlf ? (uint64_t)n * 8 : 0);
     out.build_wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_host0).count();
 
 done:

@@ -72,8 +72,9 @@ struct DeviceGraph {
     // [n * groups + 1] row pointers by label group (WalkGraph::rowgrp); the
     // row pointers themselves with one group, null with more than kMaxRowGroups
     uint32_t *rowgrp = nullptr;
-    uint64_t *nlf = nullptr;          // [n] entries by label group, a byte each (WalkGraph::nlf); null with rowgrp
-    static constexpr uint32_t kMaxRowGroups = 8;
+    uint64_t *nlf = nullptr;          // [n] entries by label group, a byte each (WalkGraph::nlf); null with
+                                      // more than 8 groups
+    static constexpr uint32_t kMaxRowGroups = 16;
     void *block = nullptr;            // the one allocation rowptr, adj, order and elab live in
     bool symmetric = false, multi = false;
     int n_edge_labels = 0;

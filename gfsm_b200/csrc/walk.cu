@@ -12,8 +12,8 @@
 // their neighbours' labels.
 //
 // Bound: instruction issue and the latency of a round's dependent loads
-// (queue entry, row entry, row pointers by label group) at 39 warps per SM;
-// ncu on 64 grid queries: 71% issue active, DRAM 1.1 TB/s.  Before (level
+// (queue entry, row entry, row pointers by label group);
+// ncu on 64 grid queries: 60-70% issue active, DRAM 1.1 TB/s.  Before (level
 // steps) and after, whole calls: one 5-vertex query on 2,000 vertices 230 ->
 // 47 us, one 7-vertex query on the 1,400 x 1,400 grid 327 -> 97 us, 64 such
 // queries of 4-10 vertices 3.4 -> 1.4 ms, 4,096 of them from edge lists 102
@@ -29,10 +29,10 @@ namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kWarps = kWalkThreads / 32;
-// CTAs an SM runs: 40 warps at 48 registers.  A round is a chain of dependent
-// loads, so warps count: 4,096 grid queries 73.5 ms with 32 warps (64
-// registers), 69.5 with 40, 73.4 with 48 (40 registers, which spill).
-constexpr uint32_t kCtas = 10;
+// CTAs an SM runs: 32 warps at 64 registers.  40 warps (48 registers) hide
+// more latency but cost instructions: 4,096 grid queries 57.4 against 58.4
+// ms, but one 67 against 63 us, 32 edge-labelled queries 215 against 197 us.
+constexpr uint32_t kCtas = 8;
 
 // A word read back from a queue is clamped to the array it indexes before it
 // is used (here and by vertex() in walk.cuh), at no cost that could be
@@ -85,6 +85,10 @@ __device__ __forceinline__ void deal(uint32_t n, uint32_t lane, uint32_t &incl, 
     from = (__popc(first & (kFull >> (31 - lane))) - 1) & 31;
     local = lane - __shfl_sync(kFull, excl, from);
 }
+
+// Candidates in a unit that a limited pass leaves, at least: few, since the
+// search below each can be long and there are far more warps than units.
+constexpr uint32_t kUnit = 8;
 
 // LIM: a pass of a limited walk (as a run-time switch its code cost the
 // unlimited walk 12%).
@@ -319,8 +323,8 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         }
         __syncwarp();  // queue entries are read by other lanes next
     }
-    // ---- what a limited pass leaves: every queue entry as units of about 32
-    // candidates (at most 64 to an entry), whole children or parts of one slice
+    // ---- what a limited pass leaves: every queue entry as units of kUnit
+    // candidates or more (about 64 to an entry at most), whole children or parts of one slice
     if (LIM && __any_sync(kFull, left != 0)) {
         if (!a.list_out) {
             if (lane == 0) a.result->gave_up = 1;
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                 const uint32_t n = min(__shfl_sync(kFull, ents, d), kQueue);
                 for (uint32_t e = lane; e < n; e += 32) {
                     const Chunk h = q[e];
-                    const uint32_t size = max(32u, (h.w + 63) / 64);
+                    const uint32_t size = max(kUnit, (h.w + 63) / 64);
                     // children whole in groups (short slices), else one by one in parts
                     const uint32_t group = max(1u, size / max(h.z, 1u));
                     for (uint32_t at = 0; at < h.w;) {

@@ -23,7 +23,7 @@ struct WalkGraph {
     // built (many groups), rows are searched.
     const uint32_t *__restrict__ rowgrp;
     // Entries of every row by label group, a byte each (at most 255); null
-    // together with rowgrp.
+    // with more than 8 groups.
     const uint64_t *__restrict__ nlf;
     uint32_t groups;
     uint32_t single_label;

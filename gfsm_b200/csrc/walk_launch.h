@@ -12,8 +12,8 @@ constexpr int kWalkThreads = 128;
 // A limited walk (Engine::run_walk) is a few passes: a warp that has taken a
 // pass's rounds writes what is left in its queues to a list, and the next
 // pass deals the list to all warps.  What the last one leaves is not walked.
-constexpr int kWalkPasses = 3;
-constexpr uint32_t kWalkRounds[kWalkPasses] = {24, 48, 192};
+constexpr int kWalkPasses = 4;
+constexpr uint32_t kWalkRounds[kWalkPasses] = {16, 24, 32, 96};
 constexpr uint32_t kWalkListed = 1u << 18;  // units a list holds
 
 constexpr int kWalkTotals = 32;

@@ -29,11 +29,11 @@ def _counts(ctx, plans, data, monkeypatch, walked):
 
 
 @pytest.mark.parametrize("nq", [1, 2, 33, 300])
-@pytest.mark.parametrize("form", ["labels", "nine_labels", "edge_labels", "repeated", "loop"])
+@pytest.mark.parametrize("form", ["labels", "many_labels", "edge_labels", "repeated", "loop", "nine_labels"])
 def test_walk_equals_level_steps(monkeypatch, form, nq):
     ctx = gfsm_b200.GFSM(device=0, vertex_labels=1)
     g = synth.grid(40, 0.05, 0.05, seed=nq)
-    g.vlabel = synth.vlabels(g.n, 9 if form == "nine_labels" else 3, 0.0, seed=4)
+    g.vlabel = synth.vlabels(g.n, {"many_labels": 17, "nine_labels": 9}.get(form, 3), 0.0, seed=4)
     s, d = g.directed()
     lab = np.ones(len(s), np.uint32)
     if form == "edge_labels":
