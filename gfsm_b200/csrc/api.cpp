@@ -43,7 +43,10 @@ Engine *ctx_engine(gfsm_ctx *ctx, const DeviceGraph &g, gfsm_status &rc, std::st
     }
     // MEMLIMIT covers the data graph, the engine's fixed buffers and the arena.
     const uint64_t used = g.bytes + e->small_bytes;
-    const uint64_t lim_cap = ctx->lim.mem_limit > used ? ctx->lim.mem_limit - used : 0;
+    uint64_t lim_cap = ctx->lim.mem_limit > used ? ctx->lim.mem_limit - used : 0;
+    // what is derived from the graph counts as well, except where a tight
+    // limit would lose much of its arena to it
+    if (lim_cap / 4 > g.aux_bytes) lim_cap -= g.aux_bytes;
     uint64_t cap = lim_cap;
     // Free device memory is read when the arena is first sized and then every
     // 1024th call (a chance to grow): the query goes through the driver,

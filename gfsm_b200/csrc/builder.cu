@@ -27,6 +27,9 @@ namespace gfsm {
 
 namespace {
 
+constexpr uint32_t kHubRow = 512;      // the longest row from which a graph gets hub bits
+constexpr uint32_t kMaxHubs = 1u << 14;
+
 #define BCHECK(x)                                                                 \
     do {                                                                          \
         cudaError_t e_ = (x);                                                     \
@@ -124,6 +127,18 @@ __global__ void k_row_groups(const uint32_t *rowptr, const uint32_t *adj, uint32
     }
 }
 
+// Bits of the adjacency among the first `hubs` vertices, a warp per row (its
+// entries below `hubs` come first).
+__global__ void k_hub_bits(const uint32_t *rowptr, const uint32_t *adj, uint32_t hubs, uint32_t *bits) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < hubs; u += gridDim.x * blockDim.x >> 5)
+        for (uint32_t i = rowptr[u] + lane; i < rowptr[u + 1]; i += 32) {
+            const uint32_t v = adj[i];
+            if (v >= hubs) break;
+            atomicOr(&bits[(u * hubs + v) >> 5], 1u << (v & 31u));
+        }
+}
+
 inline unsigned grid_for(uint64_t n, unsigned threads) {
     uint64_t b = (n + threads - 1) / threads;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(b, 148ull * 32));
@@ -133,6 +148,9 @@ inline unsigned grid_for(uint64_t n, unsigned threads) {
 
 void free_device_graph(DeviceGraph &g) {
     if (g.block) cudaFree(g.block);
+    if (g.hub_bits) cudaFree(g.hub_bits);
+    g.hub_bits = nullptr;
+    g.hubs = 0;
     g.block = nullptr;
     g.rowptr = g.adj = g.order = g.rowgrp = nullptr;
     g.elab = nullptr;
@@ -389,8 +407,27 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
             }
         }
     }
-    out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4 + grp_words * 4 +
-                (out.nlf ? (uint64_t)n * 8 : 0);
+    out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4;
+    out.aux_bytes = grp_words * 4 + (out.nlf ? (uint64_t)n * 8 : 0);
+    // Hub adjacency as bits, where rows are long and one edge label makes a
+    // check one bit: up to 16,384 vertices (32 MB, held by L2), and no more
+    // memory than the CCSR has.
+    if (out.n_edge_labels == 1 && !vl_mode && out.max_degree >= kHubRow) {
+        uint32_t k = std::min<uint32_t>(kMaxHubs, n) & ~31u;
+        while (k > 32 && (uint64_t)k * k / 8 > out.bytes / 2) k = k / 2 & ~31u;
+        const uint64_t words = (uint64_t)k * k / 32;
+        if (k >= 32 && cudaMalloc(&out.hub_bits, words * 4) == cudaSuccess) {
+            out.hubs = k;
+            out.aux_bytes += words * 4;
+            BCHECK(cudaMemsetAsync(out.hub_bits, 0, words * 4, st));
+            k_hub_bits<<<grid_for((uint64_t)k * 32, 256), 256, 0, st>>>(out.rowptr, out.adj, k, out.hub_bits);
+            BCHECK(cudaGetLastError());
+            BCHECK(cudaStreamSynchronize(st));
+        } else {
+            cudaGetLastError();
+            out.hub_bits = nullptr;
+        }
+    }
     out.build_wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_host0).count();
 
 done:

@@ -75,6 +75,11 @@ struct DeviceGraph {
     uint64_t *nlf = nullptr;          // [n] entries by label group, a byte each (WalkGraph::nlf); null with
                                       // more than 8 groups
     static constexpr uint32_t kMaxRowGroups = 16;
+    // adjacency of the `hubs` vertices of highest degree among themselves, a
+    // bit each (row u, column v: bit u * hubs + v); one edge label, vertices
+    // in degree order, a skewed graph, else null
+    uint32_t *hub_bits = nullptr;
+    uint32_t hubs = 0;
     void *block = nullptr;            // the one allocation rowptr, adj, order and elab live in
     bool symmetric = false, multi = false;
     int n_edge_labels = 0;
@@ -89,7 +94,8 @@ struct DeviceGraph {
     // degree-descending), for delta < kCutDeltas
     static constexpr uint32_t kCutDeltas = 17;
     std::vector<uint32_t> deg_cut;
-    uint64_t bytes = 0;
+    uint64_t bytes = 0;               // the CCSR (rowptr, adj, order, elab)
+    uint64_t aux_bytes = 0;           // what is derived from it (rowgrp, nlf, hub_bits)
     // build time: allocation, host-to-device copies, device passes, copies
     // back (CUDA events on the build stream), and the host wall time
     double build_ms[4] = {0, 0, 0, 0};

@@ -2,7 +2,8 @@
 parents on long rows, and descending orbits against the same steps without
 them (a context with a candidate cap far above the work keeps the earlier
 form) and, for triangles, an independent counter: rows on both sides of the
-register-held length, hubs, batches whose trie nodes mix children that are
+register-held length, hubs (unlabelled, from rows of
+512 entries, checked by bits), batches whose trie nodes mix children that are
 counted with children that are not, both drivers."""
 import numpy as np
 import pytest
@@ -15,6 +16,7 @@ pytestmark = pytest.mark.gpu
 
 GRAPHS = {
     "rmat": lambda: synth.rmat(11, 20000, seed=3),
+    "hubs": lambda: synth.rmat(12, 30000, seed=3),
     "ba": lambda: synth.ba(3000, 3, seed=4),
     "hub": lambda: synth.UGraph(400, np.concatenate([np.zeros(399, np.uint32), np.arange(1, 399, dtype=np.uint32)]),
                                 np.concatenate([np.arange(1, 400, dtype=np.uint32), np.arange(2, 400, dtype=np.uint32)])),
@@ -39,7 +41,8 @@ def test_same_counts(monkeypatch, graph, labels, driver):
     got = []
     for kw in ({}, dict(max_candidates=1 << 60)):
         ctx = gfsm_b200.GFSM(device=0, vertex_labels=vl, **kw)
-        data = ctx.graph_from_edges(g.n, s, d, None, g.vlabel)
+        data = ctx.graph_from_edges(g.n, s, d, None, g.vlabel).to_device()
+        assert graph != "hubs" or data.info()["max_degree"] >= 512
         plans = ctx.prepare_queries(flat)
         batch, st = ctx.batch_count(plans, data)
         assert batch.tolist() == [ctx.match_count(p, data)[0] for p in plans]
