@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -201,19 +202,34 @@ gfsm_status gfsm_graph_load_text(gfsm_ctx *ctx, const char *path, gfsm_graph **o
 // reference's packed CCSR keeps (CCSRRelSize).
 static gfsm_status edges_to_host(uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
                                  const uint32_t *elabel, const uint32_t *vlabel, uint32_t rel_bits, HostGraph &h) {
+    // (a data graph's arrays on several threads: first-touch page faults are
+    // most of the copy's time)
     h.n = n;
-    h.src.assign(src, src + m);
-    h.dst.assign(dst, dst + m);
+    h.src.resize(m);
+    h.dst.resize(m);
     h.lab.resize(m);
+    h.vlabel.resize(n);
     const uint32_t vb = 32u - rel_bits;
-    for (uint64_t i = 0; i < m; ++i) {
-        if (src[i] >= n || dst[i] >= n) return GFSM_ERR_INVALID_DATA;
-        const uint32_t l = elabel ? elabel[i] : 1u;
-        h.lab[i] = (uint8_t)(((uint32_t)(l << vb)) >> vb);
-    }
-    h.vlabel.assign(n, 0);
-    if (vlabel) std::memcpy(h.vlabel.data(), vlabel, (uint64_t)n * 4);
-    return GFSM_OK;
+    std::atomic<bool> ok{true};
+    par_ranges(m, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+        uint32_t most = 0;
+        for (uint64_t i = lo; i < hi; ++i) {
+            most = std::max(most, std::max(src[i], dst[i]));
+            h.src[i] = src[i];
+            h.dst[i] = dst[i];
+        }
+        if (lo < hi && most >= n) ok = false;
+        if (elabel)
+            for (uint64_t i = lo; i < hi; ++i) h.lab[i] = (uint8_t)(((uint32_t)(elabel[i] << vb)) >> vb);
+        else if (lo < hi)
+            std::memset(&h.lab[lo], (int)(uint8_t)((1u << vb) >> vb), hi - lo);
+    });
+    par_ranges(n, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+        if (lo >= hi) return;
+        if (vlabel) std::memcpy(&h.vlabel[lo], vlabel + lo, (hi - lo) * 4);
+        else std::memset(&h.vlabel[lo], 0, (hi - lo) * 4);
+    });
+    return ok ? GFSM_OK : GFSM_ERR_INVALID_DATA;
 }
 
 gfsm_status gfsm_graph_from_edges(gfsm_ctx *ctx, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst,
@@ -273,17 +289,37 @@ gfsm_status gfsm_graph_download(gfsm_ctx *ctx, const gfsm_graph *g, uint32_t *ro
     if (!g->dev) return GFSM_ERR_ARG;
     const DeviceGraph &d = *g->dev;
     cudaSetDevice(d.device);
-    if (rowptr) std::memcpy(rowptr, d.h_rowptr.data(), ((uint64_t)d.n + 1) * 4);
-    if (order) std::memcpy(order, d.h_order.data(), (uint64_t)d.n * 4);
-    if (adj && d.m && cudaMemcpy(adj, d.adj, d.m * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return GFSM_ERR_CUDA;
-    if (elab && d.m) {
-        if (d.elab) {
-            if (cudaMemcpy(elab, d.elab, d.m, cudaMemcpyDeviceToHost) != cudaSuccess) return GFSM_ERR_CUDA;
-        } else {
-            std::memset(elab, (int)d.single_label, d.m);
-        }
+    // The host copies and the constant label on other threads meanwhile; the
+    // target's pages are touched first, or the device copy would fault them in
+    // one by one.
+    auto on_host = [&] {
+        auto copy = [](uint32_t *to, const uint32_t *from, uint64_t n) {
+            par_ranges(n, kCopyGrain, [=](uint64_t lo, uint64_t hi) { std::memcpy(to + lo, from + lo, (hi - lo) * 4); });
+        };
+        if (rowptr) copy(rowptr, d.h_rowptr.data(), (uint64_t)d.n + 1);
+        if (order) copy(order, d.h_order.data(), d.n);
+        if (elab && d.m && !d.elab)
+            par_ranges(d.m, 4 * kCopyGrain,
+                       [&](uint64_t lo, uint64_t hi) { std::memset(elab + lo, (int)d.single_label, hi - lo); });
+    };
+    std::thread host;
+    try {
+        host = std::thread(on_host);
+    } catch (...) {
+        on_host();
     }
-    return GFSM_OK;
+    gfsm_status rc = GFSM_OK;
+    if (adj && d.m) {
+        par_ranges(d.m, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+            for (uint64_t i = lo; i < hi; i += 1024) adj[i] = 0;
+        });
+        if (cudaMemcpy(adj, d.adj, d.m * 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = GFSM_ERR_CUDA;
+    }
+    if (rc == GFSM_OK && elab && d.m && d.elab &&
+        cudaMemcpy(elab, d.elab, d.m, cudaMemcpyDeviceToHost) != cudaSuccess)
+        rc = GFSM_ERR_CUDA;
+    if (host.joinable()) host.join();
+    return rc;
 }
 
 void gfsm_graph_destroy(gfsm_graph *g) {
@@ -333,7 +369,7 @@ static const PlanStats &plan_stats(const gfsm_graph *data) {
         if (fwd[i].first == fwd[i - 1].first) inv = false;
     st->order_invariant = inv;
     std::vector<uint32_t> lab(h.n, 0);
-    if (g->vl_mode) lab = h.vlabel;
+    if (g->vl_mode) lab.assign(h.vlabel.begin(), h.vlabel.end());
     st->labels = lab;
     std::sort(st->labels.begin(), st->labels.end());
     st->labels.erase(std::unique(st->labels.begin(), st->labels.end()), st->labels.end());

@@ -18,8 +18,10 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdio>
+#include <mutex>
 
 #include "gfsm_internal.h"
 
@@ -81,7 +83,7 @@ __global__ void k_unpack(const unsigned long long *key, uint64_t m, uint32_t bit
         unsigned long long k = key[i];
         adj[i] = (uint32_t)(k & mask);
         if (i > 0 && key[i - 1] == k) atomicOr(&flags[0], 1u);      // duplicate (u,v)
-        if (i > 0 && lab[i] != lab[0]) atomicOr(&flags[1], 1u);     // more than one label
+        if (lab && i > 0 && lab[i] != lab[0]) atomicOr(&flags[1], 1u);     // more than one label
     }
 }
 
@@ -182,7 +184,9 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
 
     char *ws = nullptr;
     uint32_t h_flags[3] = {0, 0, 0};
-    std::vector<uint32_t> group;  // per vertex, when grouping by label
+    RawVec<uint32_t> group;       // per vertex, when grouping by label
+    bool one_label = true;        // every edge label is the same: no label copies, no payload in the sort
+    std::thread touch;            // faults the host copies' pages in meanwhile
     cudaStream_t st = nullptr;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     uint32_t *d_src, *d_dst, *d_deg, *d_group, *d_inv, *d_degs, *d_val, *d_flags;
@@ -196,6 +200,24 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     uint64_t grp_words = 0;  // rowgrp's words, where it is not rowptr itself
     auto t_host0 = std::chrono::steady_clock::now();
 
+    {
+        std::atomic<bool> same{true};
+        par_ranges(m, 4 * kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+            uint8_t other = 0;
+            for (uint64_t i = lo; i < hi; ++i) other |= h.lab[i] ^ h.lab[0];
+            if (other) same = false;
+        });
+        one_label = same;
+    }
+    out.h_rowptr.resize((uint64_t)n + 1);
+    out.h_order.resize(n);
+    try {
+        touch = std::thread([&] {
+            for (uint64_t i = 0; i < out.h_rowptr.size(); i += 1024) out.h_rowptr[i] = 0;
+            for (uint64_t i = 0; i < out.h_order.size(); i += 1024) out.h_order[i] = 0;
+        });
+    } catch (...) {  // the copies fault them in
+    }
     BCHECK(cudaSetDevice(device));
     BCHECK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     for (cudaEvent_t &e : ev) BCHECK(cudaEventCreate(&e));
@@ -203,10 +225,35 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         // label value -> group (labels ascending): a table over the value
         // range when it is small (the usual case), else a sort of the values
         uint32_t mx = 0;
-        for (uint32_t v = 0; v < n; ++v) mx = std::max(mx, h.vlabel[v]);
+        std::mutex mu;
+        par_ranges(n, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+            uint32_t most = 0;
+            for (uint64_t v = lo; v < hi; ++v) most = std::max(most, h.vlabel[v]);
+            std::lock_guard<std::mutex> lk(mu);
+            mx = std::max(mx, most);
+        });
         std::vector<uint32_t> vals;
+        std::vector<uint32_t> cnt;
         group.resize(n);
-        if (mx < (1u << 22)) {
+        if (mx < 4096) {  // a table per thread: which values there are, how often
+            std::vector<uint32_t> idx((size_t)mx + 1, 0), times((size_t)mx + 1, 0);
+            par_ranges(n, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+                std::vector<uint32_t> mine((size_t)mx + 1, 0);
+                for (uint64_t v = lo; v < hi; ++v) mine[h.vlabel[v]]++;
+                std::lock_guard<std::mutex> lk(mu);
+                for (uint32_t x = 0; x <= mx; ++x) times[x] += mine[x];
+            });
+            cnt.push_back(0);
+            for (uint32_t x = 0; x <= mx; ++x)
+                if (times[x]) {
+                    idx[x] = (uint32_t)vals.size();
+                    vals.push_back(x);
+                    cnt.push_back(times[x]);
+                }
+            par_ranges(n, kCopyGrain, [&](uint64_t lo, uint64_t hi) {
+                for (uint64_t v = lo; v < hi; ++v) group[v] = idx[h.vlabel[v]];
+            });
+        } else if (mx < (1u << 22)) {
             std::vector<uint32_t> idx((size_t)mx + 1, 0);
             for (uint32_t v = 0; v < n; ++v) idx[h.vlabel[v]] = 1;
             for (uint32_t x = 0; x <= mx; ++x)
@@ -222,8 +269,10 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
             for (uint32_t v = 0; v < n; ++v)
                 group[v] = (uint32_t)(std::lower_bound(vals.begin(), vals.end(), h.vlabel[v]) - vals.begin());
         }
-        std::vector<uint32_t> cnt(vals.size() + 1, 0);
-        for (uint32_t v = 0; v < n; ++v) cnt[group[v] + 1]++;
+        if (cnt.empty()) {
+            cnt.assign(vals.size() + 1, 0);
+            for (uint32_t v = 0; v < n; ++v) cnt[group[v] + 1]++;
+        }
         for (size_t i = 0; i < vals.size(); ++i) cnt[i + 1] += cnt[i];
         out.group_value = vals;
         out.group_start = cnt;
@@ -246,6 +295,9 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     BCHECK(cub::DeviceRadixSort::SortPairs(nullptr, need, (unsigned long long *)nullptr,
                                            (unsigned long long *)nullptr, (uint8_t *)nullptr, (uint8_t *)nullptr,
                                            (int64_t)m1, 0, 2 * bits, st));
+    tmp_bytes = std::max(tmp_bytes, need);
+    BCHECK(cub::DeviceRadixSort::SortKeys(nullptr, need, (unsigned long long *)nullptr, (unsigned long long *)nullptr,
+                                          (int64_t)m1, 0, 2 * bits, st));
     tmp_bytes = std::max(tmp_bytes, need);
 
     BCHECK(cudaEventRecord(ev[0], st));
@@ -312,7 +364,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     if (m) {
         BCHECK(cudaMemcpyAsync(d_src, h.src.data(), m * 4, cudaMemcpyHostToDevice, st));
         BCHECK(cudaMemcpyAsync(d_dst, h.dst.data(), m * 4, cudaMemcpyHostToDevice, st));
-        BCHECK(cudaMemcpyAsync(d_lab, h.lab.data(), m, cudaMemcpyHostToDevice, st));
+        if (!one_label) BCHECK(cudaMemcpyAsync(d_lab, h.lab.data(), m, cudaMemcpyHostToDevice, st));
     }
     if (vl_mode && n) BCHECK(cudaMemcpyAsync(d_group, group.data(), (uint64_t)n * 4, cudaMemcpyHostToDevice, st));
     BCHECK(cudaEventRecord(ev[2], st));
@@ -335,9 +387,12 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     // 4. entries keyed (row(src), row(dst)), labels carried as values
     if (m) {
         k_edge_keys<<<grid_for(m, 256), 256, 0, st>>>(d_src, d_dst, m, d_inv, bits, d_ekey);
-        BCHECK(cub::DeviceRadixSort::SortPairs(d_tmp, tmp_bytes, d_ekey, d_ekey2, d_lab, d_lab2, (int64_t)m, 0,
-                                               2 * bits, st));
-        k_unpack<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.adj, d_lab2, d_flags);
+        if (one_label)
+            BCHECK(cub::DeviceRadixSort::SortKeys(d_tmp, tmp_bytes, d_ekey, d_ekey2, (int64_t)m, 0, 2 * bits, st));
+        else
+            BCHECK(cub::DeviceRadixSort::SortPairs(d_tmp, tmp_bytes, d_ekey, d_ekey2, d_lab, d_lab2, (int64_t)m, 0,
+                                                   2 * bits, st));
+        k_unpack<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.adj, one_label ? nullptr : d_lab2, d_flags);
         k_symmetric<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.rowptr, out.adj, d_flags);
     }
     if (grouped) {
@@ -348,8 +403,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     BCHECK(cudaGetLastError());
     BCHECK(cudaEventRecord(ev[3], st));
     BCHECK(cudaMemcpyAsync(h_flags, d_flags, 12, cudaMemcpyDeviceToHost, st));
-    out.h_rowptr.resize((uint64_t)n + 1);
-    out.h_order.resize(n);
+    if (touch.joinable()) touch.join();
     BCHECK(cudaMemcpyAsync(out.h_rowptr.data(), out.rowptr, ((uint64_t)n + 1) * 4, cudaMemcpyDeviceToHost, st));
     if (n) BCHECK(cudaMemcpyAsync(out.h_order.data(), out.order, (uint64_t)n * 4, cudaMemcpyDeviceToHost, st));
     BCHECK(cudaEventRecord(ev[4], st));
@@ -382,13 +436,6 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         out.n_edge_labels = 1;
         out.single_label = h.lab[0];
     }
-    out.rows = 0;
-    out.max_degree = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-        uint32_t d = out.h_rowptr[i + 1] - out.h_rowptr[i];
-        if (d) out.rows++;
-        out.max_degree = std::max(out.max_degree, d);
-    }
     {
         // the degree window of every (label group, degree bound < 17): a
         // query vertex's degree bound is below its query's size (at most 16)
@@ -405,6 +452,14 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
                 }
                 out.deg_cut[(size_t)gi * K + delta] = a;
             }
+        }
+        // degrees descend inside a group: the first is its largest, and its
+        // rows with an entry end at delta 1
+        out.rows = out.max_degree = 0;
+        for (uint32_t gi = 0; gi < ng; ++gi) {
+            const uint32_t glo = out.group_start[gi];
+            if (glo < out.group_start[gi + 1]) out.max_degree = std::max(out.max_degree, out.degree(glo));
+            out.rows += out.deg_cut[(size_t)gi * K + 1] - glo;
         }
     }
     out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4;
@@ -431,6 +486,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     out.build_wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_host0).count();
 
 done:
+    if (touch.joinable()) touch.join();
     if (ws) {
         cudaFreeAsync(ws, st);
         cudaStreamSynchronize(st);

@@ -1,9 +1,11 @@
 // gfsm_internal.h -- host/device structures shared inside libgfsm.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -46,6 +48,27 @@ struct NoInitAlloc : std::allocator<T> {
 template <class T>
 using RawVec = std::vector<T, NoInitAlloc<T>>;
 
+// f(lo, hi) over [0, n) cut into equal ranges, one host thread each: at least
+// `grain` items a thread, at most 16 threads (a range whose thread cannot be
+// started runs on the caller's).
+template <class F>
+void par_ranges(uint64_t n, uint64_t grain, F f) {
+    const uint64_t hw = std::min<uint64_t>(16, std::max(1u, std::thread::hardware_concurrency()));
+    const uint64_t nt = std::max<uint64_t>(1, std::min(hw, n / grain));
+    std::vector<std::thread> pool;
+    for (uint64_t t = 1; t < nt; ++t) {
+        const uint64_t lo = n * t / nt, hi = n * (t + 1) / nt;
+        try {
+            pool.emplace_back(f, lo, hi);
+        } catch (...) {
+            f(lo, hi);
+        }
+    }
+    f((uint64_t)0, n * 1 / nt);
+    for (std::thread &th : pool) th.join();
+}
+constexpr uint64_t kCopyGrain = 1ull << 19;  // items a thread is worth (a copy of 2 MB)
+
 // ---------------------------------------------------------------------------
 // Host-side graph: the parsed edge lines, labels masked to CCSRRelSize bits.
 // ---------------------------------------------------------------------------
@@ -53,7 +76,7 @@ struct HostGraph {
     uint32_t n = 0;
     RawVec<uint32_t> src, dst;        // directed entries, input order
     RawVec<uint8_t> lab;              // edge label & ((1<<CCSRRelSize)-1)
-    std::vector<uint32_t> vlabel;     // per vertex id (v lines), 0 if absent
+    RawVec<uint32_t> vlabel;          // per vertex id (v lines), 0 if absent
 };
 
 // Device CCSR.  Internal vertex ids are the reference's CCSR row order
@@ -85,8 +108,8 @@ struct DeviceGraph {
     int n_edge_labels = 0;
     bool vl_grouped = false;
     // host copies used by the planner (degree windows) and for output
-    std::vector<uint32_t> h_rowptr;   // [n+1]
-    std::vector<uint32_t> h_order;    // [n]
+    RawVec<uint32_t> h_rowptr;        // [n+1]
+    RawVec<uint32_t> h_order;         // [n]
     std::vector<uint32_t> group_value;// sorted distinct vertex label values (grouped mode)
     std::vector<uint32_t> group_start;// [groups+1]
     // degree windows: deg_cut[g * kCutDeltas + delta] = the first id of
