@@ -1109,6 +1109,8 @@ constexpr uint32_t kWalkMaxRow = 64;
 // Longer rows: the longest row's share of one label group, for which a light
 // call tries the walk (kWalkRounds rounds a warp at most, 1 to 2 us each).
 constexpr uint32_t kWalkMaxGroupRow = 1024;
+// Results of up to this many bytes the walk writes to the host itself.
+constexpr uint64_t kWalkHostBytes = 16384;
 constexpr uint64_t kWalkMinLimit = 1ull << 20;
 constexpr uint64_t kWalkMinArena = 256ull << 20;
 
@@ -1610,11 +1612,15 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     a.counts = reinterpret_cast<unsigned long long *>(ds + o_counts);
     a.result = reinterpret_cast<WalkResult *>(ds);
     a.queues = reinterpret_cast<Chunk *>(ds + total);
+    const uint64_t back = o_counts + al(w.nslots * 8ull);
+    if (back <= kWalkHostBytes) {
+        a.host = reinterpret_cast<uint4 *>(hs);
+        a.host_words = (uint32_t)(back / 16);
+    }
     ECHECK(cudaEventRecord(ev0, stream));
     ECHECK(launch_walk(a, g.elab || g.multi, limited, reinterpret_cast<Chunk *>(ds + total + queue_bytes), sm_count, stream));
     ECHECK(cudaEventRecord(ev1, stream));
-    const uint64_t back = o_counts + w.nslots * 8ull;
-    ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
+    if (!a.host) ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
     ECHECK(cudaStreamSynchronize(stream));
     const WalkResult *r = reinterpret_cast<const WalkResult *>(hs);
     bool rest = r->gave_up != 0 || r->unit < a.units;  // work that no pass took on

@@ -378,6 +378,19 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         for (uint32_t w = 0; w < kWarps; ++w) n += cta_sum[w][threadIdx.x];
         if (n) atomicAdd(&a.result->total[blockIdx.x % kWalkTotals][threadIdx.x], n);
     }
+    // ---- the last CTA to get here hands the call's results to the host
+    if (a.host && a.last) {
+        __shared__ bool mine;
+        __threadfence();  // this thread's adds, before its CTA is counted
+        __syncthreads();
+        if (threadIdx.x == 0) mine = atomicAdd(&a.result->done, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (mine) {
+            __threadfence();
+            const uint4 *const from = reinterpret_cast<const uint4 *>(a.result);
+            for (uint32_t i = threadIdx.x; i < a.host_words; i += kWalkThreads) a.host[i] = __ldcg(from + i);
+        }
+    }
 }
 
 }  // namespace
@@ -409,6 +422,7 @@ cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lis
         a.max_rounds = limited ? kWalkRounds[p] : 0;
         a.list_in = p ? list[(p - 1) & 1] : nullptr;
         a.list_out = limited && p + 1 < kWalkPasses ? list[p & 1] : nullptr;
+        a.last = p + 1 == (limited ? kWalkPasses : 1);
         const uint32_t ctas = p ? all : first;
         if (lab && limited) k_walk<true, true><<<ctas, kWalkThreads, smem, st>>>(a);
         else if (lab) k_walk<true, false><<<ctas, kWalkThreads, smem, st>>>(a);

@@ -20,6 +20,7 @@ constexpr int kWalkTotals = 32;
 
 struct WalkResult {
     unsigned long long unit;  // units handed out so far
+    uint32_t done;     // CTAs of the last pass that have finished
     uint32_t gave_up;  // the last pass left work: the counts are not complete
     uint32_t listed[kWalkPasses];  // work units each pass left to the next ...
     uint32_t taken[kWalkPasses];   // ... and how many of them that one has handed out
@@ -38,7 +39,13 @@ struct WalkArgs {
     uint32_t roots, core, node_count, sfxs;
     unsigned long long units;  // root_off[roots]
     unsigned long long *counts;  // per slot
-    WalkResult *result;
+    WalkResult *result;          // the counts follow it
+    // Where the last CTA of the call copies result and counts (pinned host
+    // memory; null: the caller copies them): a copy of a few hundred bytes is
+    // 6 us in a stream.
+    uint4 *host;
+    uint32_t host_words;         // in 16 bytes
+    uint32_t last;               // this pass is the call's last (set by launch_walk)
     Chunk *queues;            // walk_queue_bytes(core, sms) of scratch
     // limited walks only: this pass, its rounds, what the one before left,
     // where it leaves its own
