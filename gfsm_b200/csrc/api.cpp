@@ -466,7 +466,7 @@ gfsm_status gfsm_query_prepare_batch(gfsm_ctx *ctx, int nq, const uint32_t *nv, 
     const bool vl = data ? data->vl_mode : false;
     std::vector<gfsm_status> rc(nq, GFSM_OK);
     // queries are tiny: one worker per ~64 of them, up to the host's threads
-    const int hw = std::max(1u, std::thread::hardware_concurrency());
+    const int hw = host_threads();
     const int nt = std::max(1, std::min(hw, (nq + 63) / 64));
     auto work = [&](int t) {
         HostGraph h;  // reused: every field is reassigned per query, its capacity kept
@@ -525,7 +525,7 @@ void gfsm_plan_destroy_array(gfsm_plan *const *plans, int n) {
     if (!plans) return;
     // a plan is a dozen small vectors: large batches free on a few host
     // threads (a worker that cannot be started runs on this thread)
-    const int hw = std::max(1u, std::thread::hardware_concurrency());
+    const int hw = host_threads();
     const int nt = std::max(1, std::min(hw, n / 256));
     auto work = [&](int t) {
         for (int i = t; i < n; i += nt) delete plans[i];

@@ -1727,7 +1727,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         std::vector<uint32_t> lo(nq), hi(nq);
         std::vector<char> never(nq, 0);
         std::vector<gfsm_status> qrc(nq, GFSM_OK);
-        const int nt = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), nq / 512));
+        const int nt = std::max(1, std::min<int>(host_threads(), nq / 256));
         auto work = [&](int t) {
             for (int i = t; i < nq; i += nt) {
                 bool nv = false;

@@ -48,13 +48,22 @@ struct NoInitAlloc : std::allocator<T> {
 template <class T>
 using RawVec = std::vector<T, NoInitAlloc<T>>;
 
+// The host's threads, asked for once (the answer takes some 10 us).
+inline int host_threads() {
+    static const int n = std::max(1, (int)std::thread::hardware_concurrency());
+    return n;
+}
+
 // f(lo, hi) over [0, n) cut into equal ranges, one host thread each: at least
 // `grain` items a thread, at most 16 threads (a range whose thread cannot be
 // started runs on the caller's).
 template <class F>
 void par_ranges(uint64_t n, uint64_t grain, F f) {
-    const uint64_t hw = std::min<uint64_t>(16, std::max(1u, std::thread::hardware_concurrency()));
-    const uint64_t nt = std::max<uint64_t>(1, std::min(hw, n / grain));
+    if (n < 2 * grain) {  // (a query's few edges: no look at the host's threads)
+        f((uint64_t)0, n);
+        return;
+    }
+    const uint64_t nt = std::max<uint64_t>(1, std::min<uint64_t>(std::min(16, host_threads()), n / grain));
     std::vector<std::thread> pool;
     for (uint64_t t = 1; t < nt; ++t) {
         const uint64_t lo = n * t / nt, hi = n * (t + 1) / nt;
@@ -64,7 +73,7 @@ void par_ranges(uint64_t n, uint64_t grain, F f) {
             f(lo, hi);
         }
     }
-    f((uint64_t)0, n * 1 / nt);
+    f((uint64_t)0, n / nt);
     for (std::thread &th : pool) th.join();
 }
 constexpr uint64_t kCopyGrain = 1ull << 19;  // items a thread is worth (a copy of 2 MB)

@@ -406,12 +406,15 @@ cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lis
     const uint32_t smem = tuple_chunks(a.core) * 32 * 16 * kWarps;
     a.warp_chunks = queue_chunks(a.core);
     const unsigned long long warps = (unsigned long long)sms * kCtas * kWarps;
-    // A warp takes 32 units at a time, more where each warp has many; fewer
-    // than 32 where there is not enough for all of them, so that a small
-    // call's roots spread over the whole chip.
+    // A warp takes 32 units at a time, up to 256 where each warp has many.
+    // With fewer than that each takes its share at once, so that a small
+    // call's roots spread over the whole chip; up to 128 under one root node
+    // (3.2 takes a warp of 32 left some of them a fourth: one grid query 66
+    // -> 57 us), but not under several, whose trees differ (32 edge-labelled
+    // queries 205 -> 288 us).
     unsigned long long chunk = a.units / (warps * 16) / 32 * 32;
     chunk = std::min<unsigned long long>(limited ? 32 : 256, std::max<unsigned long long>(chunk, 32));
-    if (a.units < warps * 32) chunk = std::max<unsigned long long>(1, (a.units + warps - 1) / warps);
+    if (a.units < warps * (limited || a.roots > 1 ? 32 : 128)) chunk = std::max<unsigned long long>(1, (a.units + warps - 1) / warps);
     a.chunk = (uint32_t)chunk;
     const unsigned long long need = (a.units + chunk - 1) / chunk;
     const uint32_t all = (uint32_t)sms * kCtas;

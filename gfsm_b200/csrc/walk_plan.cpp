@@ -279,7 +279,7 @@ bool build_walk(const std::vector<WalkQuery> &ws, const DeviceGraph &g, bool sha
         root[i] = {w.lo, w.hi};
     }
     // the queries one by one: a few host threads for a large batch
-    const int nt = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), (int)(nq / 256)));
+    const int nt = std::max(1, std::min<int>(host_threads(), (int)(nq / 128)));
     std::vector<char> fits(nt, 1);
     auto work = [&](int t) {
         for (uint32_t i = (uint32_t)t; i < nq; i += (uint32_t)nt)
