@@ -1543,7 +1543,7 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
                              const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
                              const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
                              const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, bool limited,
-                             std::string &err) {
+                             uint32_t *rows_out, uint64_t max_rows, uint64_t *n_rows, std::string &err) {
     ran = false;
     const uint32_t na = (uint32_t)active.size();
     const bool vl_on = lim.vertex_labels != 0;
@@ -1563,7 +1563,7 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     // larger id" extends low-degree vertices by higher-degree ones and never
     // enumerates a hub's row; a partitioned call keeps the ascending order,
     // whose parts its callers have seen.
-    if (!build_walk(ws, g, na >= 2 && !(shr && *shr == '0'), !g.multi, !limited, nparts == 1, w)) return GFSM_OK;
+    if (!build_walk(ws, g, na >= 2 && !(shr && *shr == '0'), !g.multi && !rows_out, !limited, nparts == 1, w)) return GFSM_OK;
     auto al = [](uint64_t b) { return (b + 255) & ~255ull; };
     // an entry's candidates (a row's slice for each child node) stay below
     // 2^22, so that the walk's quotients and sums over a queue are exact
@@ -1578,7 +1578,9 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     // a call whose plans the level steps would refuse for MEMLIMIT stays theirs
     const uint64_t level_head = 2ull * (na * (sizeof(DQuery) + 64ull) + (1ull << 20) * MAXQ);
     const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count), list_bytes = limited ? walk_list_bytes(w.core) : 0;
-    if (std::max(total + queue_bytes + list_bytes, level_head) > arena_cap / 2) return GFSM_OK;
+    const uint64_t rows_bytes = rows_out ? max_rows * (uint64_t)dq[0].k * 4 : 0;
+    if (max_rows >= (1ull << 32) || std::max(total + queue_bytes + list_bytes + rows_bytes, level_head) > arena_cap / 2)
+        return GFSM_OK;
     ran = true;
     gfsm_status rc = ensure_arena(arena_cap, err);
     if (rc != GFSM_OK) return rc;
@@ -1612,6 +1614,14 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     a.counts = reinterpret_cast<unsigned long long *>(ds + o_counts);
     a.result = reinterpret_cast<WalkResult *>(ds);
     a.queues = reinterpret_cast<Chunk *>(ds + total);
+    if (rows_out) {
+        a.rows = reinterpret_cast<uint32_t *>(ds + total + queue_bytes + list_bytes);
+        a.rows_ctr = rows_ctr;
+        a.order = g.order;
+        a.max_rows = max_rows;
+        std::memcpy(a.col, dq[0].col, sizeof(a.col));
+        ECHECK(cudaMemsetAsync(rows_ctr, 0, 4, stream));
+    }
     const uint64_t back = o_counts + al(w.nslots * 8ull);
     if (back <= kWalkHostBytes) {
         a.host = reinterpret_cast<uint4 *>(hs);
@@ -1634,6 +1644,15 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
         counts_out[active[i]] = cnt[w.slot[i]] * w.mult[i];
         st.count += counts_out[active[i]];
     }
+    if (rows_out) {
+        const uint64_t rows = std::min<uint64_t>(st.count, max_rows);
+        if (rows) {
+            ECHECK(cudaMemcpyAsync(rows_out, a.rows, rows * dq[0].k * 4, cudaMemcpyDeviceToHost, stream));
+            ECHECK(cudaStreamSynchronize(stream));
+        }
+        st.d2h_bytes = rows * dq[0].k * 4;
+        if (n_rows) *n_rows = rows;
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     st.kernel_ms = st.device_ms = ms;
@@ -1646,7 +1665,7 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     }
     st.peak_frontier_bytes = std::min<uint64_t>(st.peak_frontier_bytes, arena_cap);
     st.h2d_bytes = total;
-    st.d2h_bytes = back;
+    st.d2h_bytes += back;
     st.driver = 2;
     return GFSM_OK;
 }
@@ -1688,7 +1707,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     // Data with longer rows whose label groups still are short has the walk
     // try light calls (below).
     const bool short_rows = g.max_degree <= kWalkMaxRow;
-    const bool walk = variant < 0 && !rows_out && !trace && roomy && tune_driver < 0 && !env_drv &&
+    const bool walk = variant < 0 && (!rows_out || short_rows) && !trace && roomy && tune_driver < 0 && !env_drv &&
                       !env_set("GFSM_TILE") && !env_set("GFSM_SURVIVOR_GUESS") &&
                       (short_rows || g.max_degree <= kWalkMaxGroupRow * g.group_value.size());
     // The same calls' level steps count every last vertex they can at its
@@ -1798,7 +1817,8 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         bool ran = false;
         gfsm_status rc = GFSM_OK;
         if (short_rows) {
-            rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, false, err);
+            rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, false,
+                          rows_out, max_rows, n_rows, err);
         } else {
             uint64_t entries = 0;
             for (uint32_t i = 0; i < na && entries <= kGraphRootEntries; ++i)
@@ -1808,7 +1828,8 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
                 if (skip.left) {
                     --skip.left;
                 } else {
-                    rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, true, err);
+                    rc = run_walk(plans, active, dq, rlo, rhi, sym_ok, nparts, g, lim, counts_out, st, ran, true,
+                                  nullptr, 0, nullptr, err);
                     if (ran) {
                         skip.next = 8;
                     } else if (rc == GFSM_OK) {

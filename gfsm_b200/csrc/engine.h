@@ -71,7 +71,7 @@ struct Engine {
                          const std::vector<DQuery> &dq, const std::vector<uint32_t> &rlo,
                          const std::vector<uint32_t> &rhi, bool sym_ok, uint32_t nparts, const DeviceGraph &g,
                          const gfsm_limits &lim, uint64_t *counts_out, gfsm_stats &st, bool &ran, bool limited,
-                         std::string &err);
+                         uint32_t *rows_out, uint64_t max_rows, uint64_t *n_rows, std::string &err);
     int pick_variant(const std::vector<const Plan *> &plans, const DeviceGraph &g, const gfsm_limits &lim,
                      std::string &err);
     std::map<uint64_t, int> tuned;  // autotuner: workload class -> tile geometry

@@ -92,7 +92,8 @@ constexpr uint32_t kUnit = 8;
 
 // LIM: a pass of a limited walk (as a run-time switch its code cost the
 // unlimited walk 12%).
-template <bool LAB, bool LIM>
+// ROWS: mappings are written (their tables have no suffixes).
+template <bool LAB, bool LIM, bool ROWS>
 __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) {
     extern __shared__ __align__(16) uint32_t sh[];
     __shared__ unsigned long long cta_sum[kWarps][4];
@@ -284,7 +285,15 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         kept += go;
         if (go) {
             t.append(d, v);
-            if (w1.w >> 24) add(w0.w, 1);
+            if (w1.w >> 24) {
+                add(w0.w, 1);
+                if constexpr (ROWS) {
+                    const uint32_t slot = atomicAdd(a.rows_ctr, 1u);
+                    if (slot < a.max_rows)
+                        for (uint32_t x = 0; x <= d; ++x)
+                            a.rows[(size_t)slot * (d + 1) + a.col[x]] = __ldg(a.order + vertex(a.g, t[x]));
+                }
+            }
         } else {
             w0.y = 0;
         }
@@ -427,10 +436,12 @@ cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lis
         a.list_out = limited && p + 1 < kWalkPasses ? list[p & 1] : nullptr;
         a.last = p + 1 == (limited ? kWalkPasses : 1);
         const uint32_t ctas = p ? all : first;
-        if (lab && limited) k_walk<true, true><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (lab) k_walk<true, false><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (limited) k_walk<false, true><<<ctas, kWalkThreads, smem, st>>>(a);
-        else k_walk<false, false><<<ctas, kWalkThreads, smem, st>>>(a);
+        if (a.rows && lab) k_walk<true, false, true><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (a.rows) k_walk<false, false, true><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (lab && limited) k_walk<true, true, false><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (lab) k_walk<true, false, false><<<ctas, kWalkThreads, smem, st>>>(a);
+        else if (limited) k_walk<false, true, false><<<ctas, kWalkThreads, smem, st>>>(a);
+        else k_walk<false, false, false><<<ctas, kWalkThreads, smem, st>>>(a);
     }
     return cudaGetLastError();
 }

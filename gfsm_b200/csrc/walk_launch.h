@@ -46,6 +46,13 @@ struct WalkArgs {
     uint4 *host;
     uint32_t host_words;         // in 16 bytes
     uint32_t last;               // this pass is the call's last (set by launch_walk)
+    // mappings of a lone query (null: counts only): up to max_rows rows of k
+    // original vertex ids, tuple position i in column col[i]
+    uint32_t *rows;
+    uint32_t *rows_ctr;
+    const uint32_t *order;
+    unsigned long long max_rows;
+    uint8_t col[MAXQ];
     Chunk *queues;            // walk_queue_bytes(core, sms) of scratch
     // limited walks only: this pass, its rounds, what the one before left,
     // where it leaves its own
