@@ -1546,6 +1546,7 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
                              uint32_t *rows_out, uint64_t max_rows, uint64_t *n_rows, std::string &err) {
     ran = false;
     const uint32_t na = (uint32_t)active.size();
+    if (na > (1u << 20)) return GFSM_OK;  // the tables' host memory is bounded (about 1 KB a query)
     const bool vl_on = lim.vertex_labels != 0;
     std::vector<WalkQuery> ws(na);
     for (uint32_t i = 0; i < na; ++i) {

@@ -83,10 +83,13 @@ typedef struct {
     uint64_t expansions;         /* partial mappings produced, all levels          */
     uint64_t candidates;         /* candidates examined, all levels                */
     uint64_t alg_bytes;          /* algorithmic bytes (parent tuples + backward-neighbour rows + child tuples) */
-    uint64_t steps;              /* frontier steps launched                        */
+    uint64_t steps;              /* frontier steps launched (driver 2: kernels)    */
     uint64_t retries;            /* steps re-run with a smaller chunk              */
     uint64_t peak_frontier_bytes;/* most device bytes of partial mappings held at once
-                                    (measured: the live depth buffers after each step) */
+                                    (measured: the live depth buffers after each step; with
+                                    driver 2, which holds a bounded queue per warp, the bytes
+                                    whole levels would have held: every partial mapping it
+                                    extended) */
     double   kernel_ms;          /* device time of the level-step kernels (sum)    */
     double   device_ms;          /* device timeline of the call: first step to last */
     double   wall_ms;            /* host wall time of the call                     */
