@@ -1107,7 +1107,7 @@ const void *slot_kernel(int s, int ggeo, int kind) {
 // bounds (max_soln_size, max_scan_size) and the least arena.
 constexpr uint32_t kWalkMaxRow = 64;
 // Longer rows: the longest row's share of one label group, for which a light
-// call tries the walk (kWalkRounds rounds a warp at most, 1 to 2 us each).
+// call tries the walk (the passes' rounds, 168 a warp at most, 1 to 2 us each).
 constexpr uint32_t kWalkMaxGroupRow = 1024;
 // Results of up to this many bytes the walk writes to the host itself.
 constexpr uint64_t kWalkHostBytes = 16384;
@@ -1694,8 +1694,9 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     const bool env_drv = drv && *drv;
     const bool force_graph = !trace && ((env_drv && !strcmp(drv, "graph")) || (!env_drv && tune_driver == 1));
     const bool force_host = trace || (env_drv && strcmp(drv, "graph")) || (!env_drv && tune_driver == 0);
-    // The walk (walk.cu) takes counting calls on data of short rows: one lane
-    // per partial mapping is balanced there, and no level is written.  A call
+    // The walk (walk.cu) takes counting calls, and a lone query's mappings,
+    // on data of short rows: no level is written, and a lane's row scans are
+    // short (one grid query 294 -> 96 us, 4,096 of them 103 -> 62 ms).  A call
     // that names a level-step setting, caps its candidates or bounds its
     // levels tightly gets the level steps, whose schedule those settings
     // describe.

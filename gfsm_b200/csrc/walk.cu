@@ -14,10 +14,10 @@
 // Bound: instruction issue and the latency of a round's dependent loads
 // (queue entry, row entry, row pointers by label group);
 // ncu on 64 grid queries: 60-70% issue active, DRAM 1.1 TB/s.  Before (level
-// steps) and after, whole calls: one 5-vertex query on 2,000 vertices 230 ->
-// 47 us, one 7-vertex query on the 1,400 x 1,400 grid 327 -> 97 us, 64 such
+// steps) and after, whole calls: one 5-vertex query on 2,000 vertices 208 ->
+// 42 us, one 7-vertex query on the 1,400 x 1,400 grid 294 -> 96 us, 64 such
 // queries of 4-10 vertices 3.4 -> 1.4 ms, 4,096 of them from edge lists 102
-// -> 59 ms (kernel 56 ms).  One lane per search (no queues) left 9 of 32
+// -> 62 ms (kernel 57 ms).  One lane per search (no queues) left 9 of 32
 // lanes active: 4,096 queries took 507 ms.
 #include <cuda_runtime.h>
 
