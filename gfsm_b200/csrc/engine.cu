@@ -1537,6 +1537,25 @@ int Engine::pick_variant(const std::vector<const Plan *> &plans, const DeviceGra
     return best;
 }
 
+// Every later vertex a leaf of the first, with nothing to check but its edge,
+// in label groups that are the same or do not meet: a suffix always holds it.
+inline bool is_star(const DQuery &q) {
+    if (q.k < 2) return false;
+    uint32_t groups = 0;
+    for (uint32_t d = 1; d < q.k; ++d) {
+        const DLevel &L = q.lv[d];
+        if (L.nreq || L.anchor_check || L.anchor) return false;
+        bool seen = false;
+        for (uint32_t e = 1; e < d && !seen; ++e) {
+            const DLevel &M = q.lv[e];
+            seen = M.lo == L.lo && M.hi == L.hi && M.anchor_lab == L.anchor_lab;
+            if (!seen && M.lo < L.hi && L.lo < M.hi) return false;
+        }
+        groups += seen ? 0 : 1;
+    }
+    return groups <= kSfxGroups;
+}
+
 // The walk over the active queries of a call.  ran = false: the tables do
 // not hold these plans (or the arena the tables), the level steps run.
 gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::vector<int> &active,
@@ -1709,8 +1728,9 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     // Data with longer rows whose label groups still are short has the walk
     // try light calls (below).
     const bool short_rows = g.max_degree <= kWalkMaxRow;
-    const bool walk = variant < 0 && (!rows_out || short_rows) && !trace && roomy && tune_driver < 0 && !env_drv &&
-                      !env_set("GFSM_TILE") && !env_set("GFSM_SURVIVOR_GUESS") &&
+    const bool own_choice = !trace && roomy && tune_driver < 0 && !env_drv && !env_set("GFSM_TILE") &&
+                            !env_set("GFSM_SURVIVOR_GUESS");
+    const bool walk = variant < 0 && (!rows_out || short_rows) && own_choice &&
                       (short_rows || g.max_degree <= kWalkMaxGroupRow * g.group_value.size());
     // The same calls' level steps count every last vertex they can at its
     // parent, take candidates from the shortest row and, where symmetry is
@@ -1718,7 +1738,6 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     // run_walk); others examine the candidates they always did, which a
     // candidate cap counts and tight limits cut into steps.
     const bool desc = roomy && nparts == 1;
-    if (variant < 0 && !walk) variant = (plans.size() <= 1) ? 0 : pick_variant(plans, g, lim, err);
     auto t_start = std::chrono::steady_clock::now();
     const int nq = (int)plans.size();
     gfsm_stats st{};
@@ -1815,6 +1834,66 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
         err = "a data row of " + std::to_string(g.max_degree) + " entries exceeds the level step's 32-bit slice sums";
         return GFSM_ERR_TOO_LARGE;
     }
+    // Stars: a query whose other vertices all hang on its first one is counted
+    // at that vertex from its row's label groups, whatever the row's length,
+    // so its walk is bounded by the root window; the level steps enumerate one
+    // of the leaves (64 three-vertex queries, most of them paths, on a
+    // labelled R-MAT 2^20: 3.1 -> 1.9 and 3.6 -> 2.7 ms, the triangles what is
+    // left).  The other queries of a batch follow in a call of their own.  A light mixed batch has the
+    // limited walk try it whole first.
+    if (own_choice && !short_rows && !rows_out && !g.elab && !g.multi) {
+        std::vector<const Plan *> rest;
+        std::vector<int> mine, others;
+        std::vector<uint32_t> slo, shi;
+        for (uint32_t i = 0; i < na; ++i) {
+            if (is_star(dq[i])) {
+                mine.push_back(active[i]);
+                slo.push_back(rlo[i]);
+                shi.push_back(rhi[i]);
+            } else {
+                others.push_back(active[i]);
+                rest.push_back(plans[active[i]]);
+            }
+        }
+        // a call whose plans the level steps would refuse for MEMLIMIT stays theirs
+        const uint64_t level_head = 2ull * (na * (sizeof(DQuery) + 64ull) + (1ull << 20) * MAXQ);
+        bool ran = false;
+        if (!mine.empty() && (rest.empty() || !walk) && level_head <= arena_cap / 2) {
+            std::vector<DQuery> sq;
+            sq.reserve(mine.size());
+            for (uint32_t i = 0; i < na; ++i)
+                if (is_star(dq[i])) sq.push_back(dq[i]);
+            gfsm_status rc = run_walk(plans, mine, sq, slo, shi, sym_ok, nparts, g, lim, counts_out, st, ran, false,
+                                      nullptr, 0, nullptr, err);
+            if (rc != GFSM_OK) return rc;
+        }
+        if (ran) {
+            gfsm_status rc = GFSM_OK;
+            if (!rest.empty()) {
+                std::vector<uint64_t> counts(rest.size());
+                gfsm_stats r{};
+                rc = run(rest, g, lim, counts.data(), &r, nullptr, 0, nullptr, err, variant, part, nparts);
+                for (size_t i = 0; i < rest.size(); ++i) counts_out[others[i]] = counts[i];
+                r.count += st.count;
+                r.kernel_ms += st.kernel_ms;
+                r.device_ms += st.device_ms;
+                r.steps += st.steps;
+                r.launches += st.launches;
+                r.candidates += st.candidates;
+                r.expansions += st.expansions;
+                r.alg_bytes += st.alg_bytes;
+                r.peak_frontier_bytes = std::max(r.peak_frontier_bytes, st.peak_frontier_bytes);
+                r.h2d_bytes += st.h2d_bytes;
+                r.d2h_bytes += st.d2h_bytes;
+                st = r;
+            }
+            st.wall_ms =
+                std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
+            if (stats) *stats = st;
+            return rc;
+        }
+    }
+    if (variant < 0 && !walk) variant = (plans.size() <= 1) ? 0 : pick_variant(plans, g, lim, err);
     if (walk) {
         bool ran = false;
         gfsm_status rc = GFSM_OK;

@@ -241,6 +241,9 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                     const uint32_t nleaf = __ldg(&sx->nleaf);
                     if (nleaf > 1 && first) front += (uint32_t)tuple_bytes(nc - 1);
                     if (nleaf > 2) front += first * (uint32_t)tuple_bytes(nc);
+                    // a hub's row is added for each of its suffixes, under 2^29 at a time
+                    bytes = min(bytes, 1u << 31);
+                    front = min(front, 1u << 31);
                 }
                 __syncwarp();
                 continue;
