@@ -304,7 +304,8 @@ gfsm_status gfsm_graph_download(gfsm_ctx *ctx, const gfsm_graph *g, uint32_t *ro
     };
     std::thread host;
     try {
-        host = std::thread(on_host);
+        if (d.m < kThreadPays) on_host();
+        else host = std::thread(on_host);
     } catch (...) {
         on_host();
     }

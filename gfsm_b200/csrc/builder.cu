@@ -211,7 +211,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     }
     out.h_rowptr.resize((uint64_t)n + 1);
     out.h_order.resize(n);
-    try {
+    if (n >= kThreadPays) try {
         touch = std::thread([&] {
             for (uint64_t i = 0; i < out.h_rowptr.size(); i += 1024) out.h_rowptr[i] = 0;
             for (uint64_t i = 0; i < out.h_order.size(); i += 1024) out.h_order[i] = 0;

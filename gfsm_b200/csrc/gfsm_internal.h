@@ -76,6 +76,8 @@ void par_ranges(uint64_t n, uint64_t grain, F f) {
     f((uint64_t)0, n / nt);
     for (std::thread &th : pool) th.join();
 }
+// Words a helper thread's work needs to be worth its start (30-50 us).
+constexpr uint64_t kThreadPays = 1ull << 17;
 constexpr uint64_t kCopyGrain = 1ull << 19;  // items a thread is worth (a copy of 2 MB)
 
 // ---------------------------------------------------------------------------
