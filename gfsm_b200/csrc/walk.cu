@@ -422,11 +422,19 @@ cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lis
     // With fewer than that each takes its share at once, so that a small
     // call's roots spread over the whole chip; up to 128 under one root node
     // (3.2 takes a warp of 32 left some of them a fourth: one grid query 66
-    // -> 57 us), but not under several, whose trees differ (32 edge-labelled
-    // queries 205 -> 288 us).
+    // -> 57 us).  Under several, whose trees differ, each takes eight times,
+    // 8 units at least (a take costs about 10 ns of the counter): against 32
+    // or its share at once, kernel times of 32 edge-labelled queries 207 ->
+    // 179 us, 275 on a small grid 200 -> 143 us, 1,179 on a larger one 1.35
+    // -> 1.12 ms; one at a time three to twelve times as long.
     unsigned long long chunk = a.units / (warps * 16) / 32 * 32;
     chunk = std::min<unsigned long long>(limited ? 32 : 256, std::max<unsigned long long>(chunk, 32));
-    if (a.units < warps * (limited || a.roots > 1 ? 32 : 128)) chunk = std::max<unsigned long long>(1, (a.units + warps - 1) / warps);
+    const unsigned long long share = std::max<unsigned long long>(1, (a.units + warps - 1) / warps);
+    if (!limited && a.roots > 1) {
+        if (share < 256) chunk = std::min(share, std::max<unsigned long long>(8, share / 8));
+    } else if (a.units < warps * (limited ? 32 : 128)) {
+        chunk = share;
+    }
     a.chunk = (uint32_t)chunk;
     const unsigned long long need = (a.units + chunk - 1) / chunk;
     const uint32_t all = (uint32_t)sms * kCtas;
