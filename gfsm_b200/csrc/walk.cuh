@@ -55,9 +55,23 @@ struct Tuple {
     }
 };
 
-// A vertex of a tuple read back from a queue, kept inside the graph's arrays
-// whatever the queue holds.
-GFSM_HD uint32_t vertex(const WalkGraph &g, uint32_t u) { return u < g.n ? u : 0u; }
+// Told whether a clamp acts, which none should: the host test of the kernel
+// counts them.
+#ifndef GFSM_CLAMPED
+#define GFSM_CLAMPED(acts)
+#endif
+
+// A word read back from a queue, kept inside the array it indexes whatever
+// the queue holds.
+GFSM_HD uint32_t within(uint32_t x, uint32_t last) {
+    GFSM_CLAMPED(x > last);
+    return x < last ? x : last;
+}
+// A vertex of a tuple read back from a queue.
+GFSM_HD uint32_t vertex(const WalkGraph &g, uint32_t u) {
+    GFSM_CLAMPED(u >= g.n);
+    return u < g.n ? u : 0u;
+}
 
 // Rows of up to kWalkScan entries are read whole, with independent loads;
 // longer ones are searched.

@@ -1,6 +1,6 @@
 // walk.h -- the walk: a call's whole search as one kernel, each lane running
-// its own depth-first enumeration (device code in walk.cu, host tables in
-// walk_plan.cpp).  Compiled by the host compiler too (tests of the tables).
+// its own depth-first enumeration (device code in walk_kernel.cuh, host tables
+// in walk_plan.cpp).  Compiled by the host compiler too (tests of the tables).
 #pragma once
 #include <cstdint>
 #include <memory>

@@ -1,0 +1,456 @@
+// walk_kernel.cuh -- a call's whole search as one kernel.
+//
+// The level steps (engine.cu) write every partial mapping of a level to HBM
+// and read it back at the next, find a candidate's parent by binary search,
+// and pay several launches per level.  Where rows are short (road-like and
+// bounded-degree graphs) a parent has about one candidate, and that work is
+// several times the check itself: 23 warp instructions per candidate.  Here
+// every warp searches depth first over its own small queues, one per depth,
+// and nothing leaves the chip's caches but counts.  Prefixes are shared
+// through the same trie as in the level steps; trailing leaves are counted
+// without being enumerated (walk.cuh); a batch's vertices are filtered by
+// their neighbours' labels.
+//
+// Bound: instruction issue and the latency of a round's dependent loads
+// (queue entry, row entry, row pointers by label group);
+// ncu on 64 grid queries: 60-70% issue active, DRAM 1.1 TB/s.  Before (level
+// steps) and after, whole calls: one 5-vertex query on 2,000 vertices 208 ->
+// 42 us, one 7-vertex query on the 1,400 x 1,400 grid 294 -> 96 us, 64 such
+// queries of 4-10 vertices 3.4 -> 1.4 ms, 4,096 of them from edge lists 102
+// -> 62 ms (kernel 57 ms).  One lane per search (no queues) left 9 of 32
+// lanes active: 4,096 queries took 507 ms.
+//
+// Compiled by the host compiler too, with 32-lane stand-ins for the warp
+// intrinsics (the test that runs every lane of it in a random order).
+#pragma once
+#include "walk_launch.h"
+
+namespace gfsm {
+
+namespace {
+
+#ifdef __CUDACC__
+#define GFSM_DYN_SHARED(x) extern __shared__ __align__(16) uint32_t x[]
+#endif
+
+constexpr uint32_t kFull = 0xffffffffu;
+constexpr uint32_t kWarps = kWalkThreads / 32;
+// CTAs an SM runs: 32 warps at 64 registers.  40 warps (48 registers) hide
+// more latency but cost instructions: 4,096 grid queries 57.4 against 58.4
+// ms, but one 67 against 63 us, 32 edge-labelled queries 215 against 197 us.
+constexpr uint32_t kCtas = 8;
+
+// A word read back from a queue or a list is clamped to the array it indexes
+// before it is used (within() and vertex() in walk.cuh, place() here), at no
+// cost that could be measured: no access leaves its array whatever a queue
+// holds.  The host test of this kernel asserts that no clamp ever acts.
+//
+// A queue holds the partial mappings of one depth whose candidates are still
+// to be checked.  A round takes 32 candidates of the deepest depth that has
+// so many, so every deeper queue holds fewer than 32 entries (each has a
+// candidate at least) and takes the round's up to 32 children: 63 at most.
+constexpr uint32_t kQueue = 64;
+// An entry is 16-byte chunks (each kQueue apart): a header -- the children's
+// first node, slice start, slice length, candidates left -- and the tuple.
+// Tuples whose suffixes are still to be counted have a queue of their own,
+// emptied down to 31 pairs before any other round (header: first suffix,
+// tuple length, -, suffixes left).
+__host__ __device__ constexpr uint32_t tuple_chunks(uint32_t n) { return (n + 3) / 4; }
+// An entry's place in its queue (63 entries at most, see above).
+__device__ __forceinline__ uint32_t place(uint32_t e) {
+    GFSM_CLAMPED(e >= kQueue);
+    return e % kQueue;
+}
+// Chunks before depth d's queue (d >= 1; its entries have d vertices).
+__host__ __device__ constexpr uint32_t queue_base(uint32_t d) {
+    // sum over x < d of 1 + ceil(x / 4): four depths to each chunk count
+    const uint32_t f = (d - 1) / 4, r = (d - 1) % 4;
+    return kQueue * ((d - 1) + 2 * f * (f + 1) + r * (f + 1));
+}
+static_assert(queue_base(1) == 0 && queue_base(2) == 2 * kQueue && queue_base(6) == 11 * kQueue, "queue layout");
+// Chunks of one warp's queues: depths 1 .. core - 1, then the suffix queue.
+__host__ __device__ constexpr uint32_t queue_chunks(uint32_t core) {
+    return queue_base(core) + kQueue * (1 + tuple_chunks(core));
+}
+
+__device__ __forceinline__ unsigned long long warp_total(unsigned long long x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+    return x;
+}
+
+// Deals 32 items to 32 lanes: lane i brings n items, lane l gets item `local`
+// of lane `from` (the first 32 items in lane order).  incl: running total.
+// The lanes that bring any come before those that bring none.
+__device__ __forceinline__ void deal(uint32_t n, uint32_t lane, uint32_t &incl, uint32_t &total, uint32_t &from,
+                                     uint32_t &local) {
+    incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    total = __shfl_sync(kFull, incl, 31);
+    const uint32_t excl = incl - n;
+    // the bits where a lane's items start; from = how many started before
+    const uint32_t first = __reduce_or_sync(kFull, n && excl < 32 ? 1u << excl : 0u);
+    from = (__popc(first & (kFull >> (31 - lane))) - 1) & 31;
+    local = lane - __shfl_sync(kFull, excl, from);
+}
+
+// Candidates in a unit that a limited pass leaves, at least: few, since the
+// search below each can be long and there are far more warps than units.
+constexpr uint32_t kUnit = 8;
+
+// LIM: a pass of a limited walk (as a run-time switch its code cost the
+// unlimited walk 12%).
+// ROWS: mappings are written (their tables have no suffixes).
+template <bool LAB, bool LIM, bool ROWS>
+__global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) {
+    GFSM_DYN_SHARED(sh);  // walk_smem() bytes
+    __shared__ unsigned long long cta_sum[kWarps][4];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const Tuple t{sh + (warp * tuple_chunks(a.core) * 32 + lane) * 4, 128};  // this lane's candidate's tuple
+    Chunk *const queues = a.queues + (size_t)(blockIdx.x * kWarps + warp) * a.warp_chunks;
+    Chunk *const squeue = queues + queue_base(a.core);
+    uint32_t sents = 0, spairs = 0;  // the suffix queue's entries and (tuple, suffix) pairs
+    uint32_t ents = 0, left = 0;     // lane d: entries and candidates of depth d's queue,
+    const uint32_t base = queue_base(max(lane, 1u));  // and where it starts
+    uint32_t fslot = 0, cand = 0, kept = 0, bytes = 0, front = 0;
+    unsigned long long fcount = 0;
+    unsigned long long u_next = 0, u_end = 0;  // this warp's units
+    bool more = true;
+    uint32_t rounds = 0;
+    // units of the list (l_end == 0: none left), dealt a few at a time
+    const uint32_t l_count = LIM && a.pass ? min(__ldcg(&a.result->listed[a.pass - 1]), kWalkListed) : 0u;
+    const uint32_t l_chunk = max(1u, min(32u, l_count / (gridDim.x * kWarps)));
+    uint32_t l_next = 1, l_end = l_count ? 1u : 0u;
+    const uint32_t unit_chunks = 1 + tuple_chunks(a.core) + 1;
+    // n units, a lane each, into the queues of their depths
+    auto take_units = [&](uint32_t first, uint32_t n) {
+        const Chunk *const u = a.list_in + (size_t)(first + lane) * unit_chunks;
+        const bool has = lane < n;
+        Chunk h{0, 0, 0, 0};
+        uint32_t d = 0;
+        if (has) {
+            h = u[0];
+            d = max(within(u[1].x, a.core - 1), 1u);
+        }
+        for (uint32_t rest = __ballot_sync(kFull, has); rest;) {
+            const uint32_t depth = __shfl_sync(kFull, d, __ffs(rest) - 1);
+            const uint32_t same = __ballot_sync(kFull, has && d == depth);
+            const uint32_t e0 = __shfl_sync(kFull, ents, depth);
+            Chunk *const q = queues + __shfl_sync(kFull, base, depth);
+            const bool mine = has && d == depth;
+            if (mine) {
+                const uint32_t e = place(e0 + __popc(same & below));
+                q[e] = h;
+                for (uint32_t x = 0; x * 4 < depth; ++x) q[(1 + x) * kQueue + e] = u[2 + x];
+            }
+            const uint32_t got = __reduce_add_sync(kFull, mine ? h.w : 0u);
+            if (lane == depth) {
+                ents = e0 + __popc(same);
+                left += got;
+            }
+            rest &= ~same;
+        }
+        __syncwarp();
+    };
+    auto add = [&](uint32_t slot, unsigned long long n) {
+        if (fslot != slot && fcount) {
+            atomicAdd(a.counts + fslot, fcount);
+            fcount = 0;
+        }
+        fslot = slot;
+        fcount += n;
+    };
+    for (;;) {
+        // ---- this round's work: suffixes once there are 32 pairs; else the
+        // deepest depth with 32 candidates; else new roots; else (no more
+        // roots) the shallowest depth with any; at last the rest of the pairs
+        const uint32_t full = __ballot_sync(kFull, left >= 32), any = __ballot_sync(kFull, left != 0);
+        uint32_t d = 0;
+        bool sfx = spairs >= 32;
+        const bool closing = LIM && ++rounds > a.max_rounds;
+        if (closing && !sfx) {
+            if (!spairs) break;
+            sfx = true;
+        }
+        if (!sfx) {
+            if (full) {
+                d = 31 - __clz(full);
+            } else {
+                if (LIM && l_end) {  // units that the pass before left come first
+                    if (l_next >= l_end) {
+                        uint32_t u = 0;
+                        if (lane == 0) {
+                            u = __ldcg(&a.result->taken[a.pass - 1]);
+                            if (u < l_count) u = atomicAdd(&a.result->taken[a.pass - 1], l_chunk);
+                        }
+                        l_next = __shfl_sync(kFull, u, 0);
+                        l_end = min(l_next + l_chunk, l_count);
+                        if (l_next >= l_count) l_next = l_end = 0;
+                    }
+                    if (l_end) {
+                        take_units(l_next, min(l_end - l_next, 32u));
+                        l_next += 32;
+                        continue;
+                    }
+                }
+                if (more && u_next >= u_end) {
+                    // (a warp's first take goes straight to the counter; later it
+                    // looks whether any are left: 5,920 warps adding to one
+                    // word just to find out took 20 us)
+                    unsigned long long u = 0;
+                    if (lane == 0) {
+                        if (u_end || (LIM && a.pass)) u = __ldcg(&a.result->unit);
+                        if (u < a.units) u = atomicAdd(&a.result->unit, (unsigned long long)a.chunk);
+                    }
+                    u_next = __shfl_sync(kFull, u, 0);
+                    u_end = min(u_next + a.chunk, a.units);
+                    more = u_next < a.units;
+                }
+                if (!more) {
+                    if (any) d = __ffs(any) - 1;
+                    else if (spairs) sfx = true;
+                    else break;
+                }
+            }
+        }
+        uint32_t c = 0, v = 0, idx = 0;
+        bool act = false;
+        if (sfx || d) {
+            // ---- 32 items from the top of a queue, dealt to the lanes
+            const uint32_t qd = __shfl_sync(kFull, base, d);
+            Chunk *const q = sfx ? squeue : queues + qd;
+            const uint32_t nd = __shfl_sync(kFull, ents, d), n = within(sfx ? sents : nd, kQueue);
+            const uint32_t rem = lane < n ? q[n - 1 - lane].w : 0;
+            uint32_t incl, total, from, local;
+            deal(rem, lane, incl, total, from, local);
+            const uint32_t take = min(total, 32u), e = n - 1 - from;
+            const uint32_t frem = __shfl_sync(kFull, rem, from);
+            act = lane < take;
+            Chunk h{0, 0, 0, 0};
+            if (act) {
+                h = q[e];
+                const uint32_t nc = sfx ? within(h.y, a.core) : d;
+                for (uint32_t x = 0; x * 4 < nc; ++x) t.chunk(x) = q[(1 + x) * kQueue + e];
+            }
+            const uint32_t gone = __popc(__ballot_sync(kFull, rem && incl <= take));
+            if (rem && incl > take && incl - rem < take) q[n - 1 - lane].w = incl - take;
+            // from the end of what the entry had left: brought along by shuffle,
+            // since the word in memory changes above (another lane's store)
+            uint32_t i = frem - 1 - local;
+            if (sfx) {
+                sents = n - gone;
+                spairs -= take;
+                if (act) {
+                    const WSfx *sx = a.sfx + within(h.x + i, a.sfxs - 1);
+                    const uint32_t nc = within(h.y, a.core);
+                    uint32_t first = 0;
+                    const unsigned long long ways = suffix_count<LAB>(a.g, sx, t, nc, bytes, first);
+                    if (ways) add(__ldg(&sx->slot), ways);
+                    const uint32_t nleaf = __ldg(&sx->nleaf);
+                    if (nleaf > 1 && first) front += (uint32_t)tuple_bytes(nc - 1);
+                    if (nleaf > 2) front += first * (uint32_t)tuple_bytes(nc);
+                    // a hub's row is added for each of its suffixes, under 2^29 at a time
+                    bytes = min(bytes, 1u << 31);
+                    front = min(front, 1u << 31);
+                }
+                __syncwarp();
+                continue;
+            }
+            if (lane == d) {
+                ents = n - gone;
+                left -= take;
+            }
+            if (act) {
+                c = h.x;
+                if (i >= h.z) {  // (child node, slice entry); the quotient is exact after one correction
+                    uint32_t j = (uint32_t)__fdividef((float)i, (float)h.z);
+                    if (j * h.z > i) --j;
+                    if (i - j * h.z >= h.z) ++j;
+                    c += j;
+                    i -= j * h.z;
+                }
+                c = within(c, a.node_count - 1);
+                idx = within(h.y + i, a.g.m - 1);
+                v = __ldg(a.g.adj + idx);
+            }
+        } else {
+            const unsigned long long u = u_next + lane;
+            act = u < u_end;
+            if (act) {
+                uint32_t lo = 0, hi = a.roots;  // largest p with root_off[p] <= u
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (__ldg(a.root_off + mid) <= u) lo = mid; else hi = mid;
+                }
+                c = lo;
+                v = __ldg(a.root_lo + lo) + (uint32_t)(u - __ldg(a.root_off + lo));
+                bytes += 4;
+            }
+            u_next = min(u_next + 32, u_end);
+        }
+        // ---- check (the node's words are fetched along with the candidate)
+        const WNode *const w = a.nodes + c;
+        uint4 w0 = __ldg(reinterpret_cast<const uint4 *>(w)), w1 = __ldg(reinterpret_cast<const uint4 *>(w) + 1);
+        const bool go = act && walk_check<LAB>(a.g, w, a.again, t, d, v, idx, bytes);
+        cand += act;
+        kept += go;
+        if (go) {
+            t.append(d, v);
+            if (w1.w >> 24) {
+                add(w0.w, 1);
+                if constexpr (ROWS) {
+                    const uint32_t slot = atomicAdd(a.rows_ctr, 1u);
+                    if (slot < a.max_rows)
+                        for (uint32_t x = 0; x <= d; ++x)
+                            a.rows[(size_t)slot * (d + 1) + a.col[x]] = __ldg(a.order + vertex(a.g, t[x]));
+                }
+            }
+        } else {
+            w0.y = 0;
+        }
+        // ---- a tuple with suffixes joins the suffix queue
+        const uint32_t nsfx = w0.y >> 16;
+        const uint32_t sput = __ballot_sync(kFull, nsfx);
+        if (sput) {
+            if (nsfx) {
+                const uint32_t e = place(sents + __popc(sput & below));
+                squeue[e] = Chunk{w0.z, d + 1, 0, nsfx};
+                for (uint32_t x = 0; x * 4 <= d; ++x) squeue[(1 + x) * kQueue + e] = t.chunk(x);
+            }
+            sents += __popc(sput);
+            spairs += __reduce_add_sync(kFull, nsfx);
+        }
+        // ---- its children's slice; what has candidates joins the next queue
+        // (a node's depth is its entry's: none below the last queue has children)
+        GFSM_CLAMPED(d + 1 >= a.core && (w0.y & 0xffffu));
+        const uint32_t nkid = d + 1 < a.core ? w0.y & 0xffffu : 0u;
+        uint32_t s = 0, len = 0;
+        if (nkid) walk_slice(a.g, Chunk{w1.x, w1.y, w1.z, w1.w}, t, s, len, bytes);
+        const uint32_t put = __ballot_sync(kFull, len != 0);
+        if (put) {
+            Chunk *const q = queues + __shfl_sync(kFull, base, d + 1);
+            const uint32_t n = __shfl_sync(kFull, ents, d + 1);
+            if (len) {
+                const uint32_t e = place(n + __popc(put & below));
+                q[e] = Chunk{w0.x, s, len, len * nkid};
+                for (uint32_t x = 0; x * 4 <= d; ++x) q[(1 + x) * kQueue + e] = t.chunk(x);
+                front += (uint32_t)tuple_bytes(d);
+                bytes += 4 * (d + 1);
+            }
+            const uint32_t got = __reduce_add_sync(kFull, len * nkid);
+            if (lane == d + 1) {
+                ents = n + __popc(put);
+                left += got;
+            }
+        }
+        __syncwarp();  // queue entries are read by other lanes next
+    }
+    // ---- what a limited pass leaves: every queue entry as units of kUnit
+    // candidates or more (about 64 to an entry at most), whole children or parts of one slice
+    if (LIM && __any_sync(kFull, left != 0)) {
+        if (!a.list_out) {
+            if (lane == 0) a.result->gave_up = 1;
+        } else {
+            for (uint32_t d = 1; d < a.core; ++d) {
+                const Chunk *const q = queues + __shfl_sync(kFull, base, d);
+                const uint32_t n = within(__shfl_sync(kFull, ents, d), kQueue);
+                for (uint32_t e = lane; e < n; e += 32) {
+                    const Chunk h = q[e];
+                    const uint32_t size = max(kUnit, (h.w + 63) / 64);
+                    // children whole in groups (short slices), else one by one in parts
+                    const uint32_t group = max(1u, size / max(h.z, 1u));
+                    for (uint32_t at = 0; at < h.w;) {
+                        const uint32_t j = at / h.z, i = at - j * h.z;
+                        Chunk u{h.x + j, h.y + i, min(min(h.z - i, size), h.w - at), 0};
+                        u.w = u.z;
+                        if (i == 0 && u.z == h.z) u.w = h.z * min(group, (h.w - at) / h.z);
+                        at += u.w;
+                        const uint32_t slot = atomicAdd(&a.result->listed[a.pass], 1u);
+                        if (slot >= kWalkListed) {
+                            a.result->gave_up = 1;
+                            break;
+                        }
+                        Chunk *const o = a.list_out + (size_t)slot * unit_chunks;
+                        o[0] = u;
+                        o[1] = Chunk{d, 0, 0, 0};
+                        for (uint32_t x = 0; x * 4 < d; ++x) o[2 + x] = q[(1 + x) * kQueue + e];
+                    }
+                }
+            }
+        }
+    }
+    // ---- counts and totals.  5,920 warps adding to the same words one by one
+    // took 25 us: a warp whose lanes hold one slot's count adds once, a CTA its
+    // totals once, to one of kWalkTotals places.
+    const uint32_t hold = __ballot_sync(kFull, fcount != 0);
+    if (hold) {
+        const uint32_t slot = __shfl_sync(kFull, fslot, __ffs(hold) - 1);
+        if (__all_sync(kFull, fcount == 0 || fslot == slot)) {
+            const unsigned long long n = warp_total(fcount);
+            if (lane == 0) atomicAdd(a.counts + slot, n);
+        } else if (fcount) {
+            atomicAdd(a.counts + fslot, fcount);
+        }
+    }
+    const unsigned long long sum[4] = {warp_total(cand), warp_total(kept), warp_total(bytes), warp_total(front)};
+    if (lane < 4) cta_sum[warp][lane] = lane < 2 ? (lane ? sum[1] : sum[0]) : (lane == 3 ? sum[3] : sum[2]);
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        unsigned long long n = 0;
+        for (uint32_t w = 0; w < kWarps; ++w) n += cta_sum[w][threadIdx.x];
+        if (n) atomicAdd(&a.result->total[blockIdx.x % kWalkTotals][threadIdx.x], n);
+    }
+    // ---- the last CTA to get here hands the call's results to the host
+    if (a.host && a.last) {
+        __shared__ bool mine;
+        __threadfence();  // this thread's adds, before its CTA is counted
+        __syncthreads();
+        if (threadIdx.x == 0) mine = atomicAdd(&a.result->done, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (mine) {
+            __threadfence();
+            const uint4 *const from = reinterpret_cast<const uint4 *>(a.result);
+            for (uint32_t i = threadIdx.x; i < a.host_words; i += kWalkThreads) a.host[i] = __ldcg(from + i);
+        }
+    }
+}
+
+// Bytes of dynamic shared memory: every lane's tuple.
+inline uint32_t walk_smem(uint32_t core) { return tuple_chunks(core) * 32 * 16 * kWarps; }
+
+// The units a warp takes at a time and the CTAs of the first pass.
+struct WalkShape {
+    uint32_t chunk, ctas;
+};
+inline WalkShape walk_shape(unsigned long long units, uint32_t roots, bool limited, int sms) {
+    const unsigned long long warps = (unsigned long long)sms * kCtas * kWarps;
+    // A warp takes 32 units at a time, up to 256 where each warp has many.
+    // With fewer than that each takes its share at once, so that a small
+    // call's roots spread over the whole chip; up to 128 under one root node
+    // (3.2 takes a warp of 32 left some of them a fourth: one grid query 66
+    // -> 57 us).  Under several, whose trees differ, each takes eight times,
+    // 8 units at least (a take costs about 10 ns of the counter): against 32
+    // or its share at once, kernel times of 32 edge-labelled queries 207 ->
+    // 179 us, 275 on a small grid 200 -> 143 us, 1,179 on a larger one 1.35
+    // -> 1.12 ms; one at a time three to twelve times as long.
+    unsigned long long chunk = units / (warps * 16) / 32 * 32;
+    chunk = std::min<unsigned long long>(limited ? 32 : 256, std::max<unsigned long long>(chunk, 32));
+    const unsigned long long share = std::max<unsigned long long>(1, (units + warps - 1) / warps);
+    if (!limited && roots > 1) {
+        if (share < 256) chunk = std::min(share, std::max<unsigned long long>(8, share / 8));
+    } else if (units < warps * (limited ? 32 : 128)) {
+        chunk = share;
+    }
+    const unsigned long long need = (units + chunk - 1) / chunk;
+    const uint32_t all = (uint32_t)sms * kCtas;
+    return {(uint32_t)chunk,
+            (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(all, (need + kWarps - 1) / kWarps))};
+}
+
+}  // namespace
+
+}  // namespace gfsm
