@@ -1597,10 +1597,13 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
                    total = o_off + al((nr + 1) * 8ull);
     // a call whose plans the level steps would refuse for MEMLIMIT stays theirs
     const uint64_t level_head = 2ull * (na * (sizeof(DQuery) + 64ull) + (1ull << 20) * MAXQ);
-    const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count), list_bytes = limited ? walk_list_bytes(w.core) : 0;
+    const uint64_t queue_bytes = walk_queue_bytes(w.core, sm_count);
     const uint64_t rows_bytes = rows_out ? max_rows * (uint64_t)dq[0].k * 4 : 0;
-    if (max_rows >= (1ull << 32) || std::max(total + queue_bytes + list_bytes + rows_bytes, level_head) > arena_cap / 2)
-        return GFSM_OK;
+    const uint64_t need = total + queue_bytes + rows_bytes;
+    // (a whole walk without room for the lists keeps each warp's work where it is)
+    uint64_t list_bytes = walk_list_bytes(w.core);
+    if (!limited && need + list_bytes > arena_cap / 2) list_bytes = 0;
+    if (max_rows >= (1ull << 32) || std::max(need + list_bytes, level_head) > arena_cap / 2) return GFSM_OK;
     ran = true;
     gfsm_status rc = ensure_arena(arena_cap, err);
     if (rc != GFSM_OK) return rc;
@@ -1647,14 +1650,29 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
         a.host = reinterpret_cast<uint4 *>(hs);
         a.host_words = (uint32_t)(back / 16);
     }
-    ECHECK(cudaEventRecord(ev0, stream));
-    ECHECK(launch_walk(a, g.elab || g.multi, limited, reinterpret_cast<Chunk *>(ds + total + queue_bytes), sm_count, stream));
-    ECHECK(cudaEventRecord(ev1, stream));
-    if (!a.host) ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
-    ECHECK(cudaStreamSynchronize(stream));
     const WalkResult *r = reinterpret_cast<const WalkResult *>(hs);
+    Chunk *const lists = list_bytes ? reinterpret_cast<Chunk *>(ds + total + queue_bytes) : nullptr;
+    int passes = 0;
+    double kernel_ms = 0;
+    // A whole walk goes on while warps have kept work, each at least
+    // kWalkLookFew rounds a pass.
+    for (uint32_t kept = 0;;) {
+        ECHECK(cudaEventRecord(ev0, stream));
+        do
+            ECHECK(launch_walk(a, g.elab || g.multi, limited, lists, passes++, kept, sm_count, stream));
+        while (limited && passes < kWalkPasses);
+        ECHECK(cudaEventRecord(ev1, stream));
+        if (!a.host) ECHECK(cudaMemcpyAsync(hs, ds, back, cudaMemcpyDeviceToHost, stream));
+        ECHECK(cudaStreamSynchronize(stream));
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ev0, ev1);
+        kernel_ms += ms;
+        kept = limited || !lists ? 0 : r->kept;
+        if (!kept) break;
+    }
     bool rest = r->gave_up != 0 || r->unit < a.units;  // work that no pass took on
-    for (int p = 0; limited && p + 1 < kWalkPasses; ++p) rest = rest || r->taken[p] < std::min(r->listed[p], kWalkListed);
+    for (int p = 0; limited && p + 1 < kWalkPasses; ++p)
+        rest = rest || r->list[p].taken < std::min(r->list[p].listed, kWalkListed);
     if (rest) {
         ran = false;
         return GFSM_OK;
@@ -1673,10 +1691,8 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
         st.d2h_bytes = rows * dq[0].k * 4;
         if (n_rows) *n_rows = rows;
     }
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev0, ev1);
-    st.kernel_ms = st.device_ms = ms;
-    st.steps = st.launches = limited ? kWalkPasses : 1;
+    st.kernel_ms = st.device_ms = kernel_ms;
+    st.steps = st.launches = (uint32_t)(limited ? passes : 2 * passes - 1);
     for (const auto &t : r->total) {
         st.candidates += t[0];
         st.expansions += t[1];

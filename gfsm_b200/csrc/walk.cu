@@ -9,29 +9,21 @@ uint64_t walk_queue_bytes(uint32_t core, int sms) {
     return (uint64_t)sms * kCtas * kWarps * queue_chunks(core) * 16;
 }
 
+// (the second list's place holds a whole walk's states)
+static_assert((uint64_t)kWalkListed * 3 * sizeof(Chunk) >= 256ull * kCtas * kWarps * sizeof(WalkState), "states");
+
 uint64_t walk_list_bytes(uint32_t core) { return 2ull * kWalkListed * (2 + tuple_chunks(core)) * 16; }
 
-cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int sms, cudaStream_t st) {
-    WalkArgs a = args;
+cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int p, uint32_t kept, int sms,
+                        cudaStream_t st) {
+    const WalkArgs a = walk_pass(args, limited, lists, p, kept, sms);
     const uint32_t smem = walk_smem(a.core);
-    a.warp_chunks = queue_chunks(a.core);
-    const WalkShape shape = walk_shape(a.units, a.roots, limited, sms);
-    a.chunk = shape.chunk;
-    Chunk *const list[2] = {lists, lists + (size_t)kWalkListed * (2 + tuple_chunks(a.core))};
-    for (int p = 0; p < (limited ? kWalkPasses : 1); ++p) {
-        a.pass = (uint32_t)p;
-        a.max_rounds = limited ? kWalkRounds[p] : 0;
-        a.list_in = p ? list[(p - 1) & 1] : nullptr;
-        a.list_out = limited && p + 1 < kWalkPasses ? list[p & 1] : nullptr;
-        a.last = p + 1 == (limited ? kWalkPasses : 1);
-        const uint32_t ctas = p ? (uint32_t)sms * kCtas : shape.ctas;
-        if (a.rows && lab) k_walk<true, false, true><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (a.rows) k_walk<false, false, true><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (lab && limited) k_walk<true, true, false><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (lab) k_walk<true, false, false><<<ctas, kWalkThreads, smem, st>>>(a);
-        else if (limited) k_walk<false, true, false><<<ctas, kWalkThreads, smem, st>>>(a);
-        else k_walk<false, false, false><<<ctas, kWalkThreads, smem, st>>>(a);
+    if (p && !limited) {
+        cudaMemsetAsync(a.out, 0, sizeof(WalkResult::List), st);
+        cudaMemsetAsync(&a.result->kept, 0, sizeof(uint32_t), st);
+        k_split<<<(a.state_warps + kWarps - 1) / kWarps, kWalkThreads, 0, st>>>(a);
     }
+    walk_kernel(a, lab, limited ? kLimited : p ? kLater : kWhole)<<<a.ctas, kWalkThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 

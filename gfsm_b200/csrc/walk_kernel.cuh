@@ -102,11 +102,28 @@ __device__ __forceinline__ void deal(uint32_t n, uint32_t lane, uint32_t &incl, 
 // search below each can be long and there are far more warps than units.
 constexpr uint32_t kUnit = 8;
 
-// LIM: a pass of a limited walk (as a run-time switch its code cost the
-// unlimited walk 12%).
+// The unit of a queue entry (header h) that starts at its candidate `at`:
+// children whole in groups where the slice is short, else parts of one slice.
+__device__ __forceinline__ Chunk unit_at(const Chunk &h, uint32_t at, uint32_t size) {
+    const uint32_t len = max(h.z, 1u), j = at / len, i = at - j * len;
+    Chunk u{h.x + j, h.y + i, min(min(len - i, size), h.w - at), 0};
+    u.w = u.z;
+    if (i == 0 && u.z == len) u.w = len * min(max(1u, size / len), (h.w - at) / len);
+    return u;  // (one candidate at least)
+}
+
+// Units in a list of which `listed` were asked for.
+__host__ __device__ inline uint32_t list_units(uint32_t listed, uint32_t refused) {
+    return listed <= kWalkListed ? listed : min(refused, kWalkListed);
+}
+
+// MODE: a whole walk's first pass, a pass of a limited walk, or a whole walk's
+// later pass (as run-time switches they cost the first pass 5-12%).
 // ROWS: mappings are written (their tables have no suffixes).
-template <bool LAB, bool LIM, bool ROWS>
+enum WalkMode { kWhole, kLimited, kLater };
+template <bool LAB, WalkMode MODE, bool ROWS>
 __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) {
+    constexpr bool LIM = MODE == kLimited;
     GFSM_DYN_SHARED(sh);  // walk_smem() bytes
     __shared__ unsigned long long cta_sum[kWarps][4];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
@@ -121,8 +138,19 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
     unsigned long long u_next = 0, u_end = 0;  // this warp's units
     bool more = true;
     uint32_t rounds = 0;
+    if (MODE == kLater && blockIdx.x * kWarps + warp < a.state_warps) {  // what this warp kept
+        const WalkState &st = a.state_in[blockIdx.x * kWarps + warp];
+        if (st.open) {
+            ents = within(st.ents[lane], kQueue - 1);
+            left = st.left[lane];
+            sents = within(st.sents, kQueue - 1);
+            spairs = st.spairs;
+            u_next = st.u_next;
+            u_end = min(st.u_end, a.units);
+        }
+    }
     // units of the list (l_end == 0: none left), dealt a few at a time
-    const uint32_t l_count = LIM && a.pass ? min(__ldcg(&a.result->listed[a.pass - 1]), kWalkListed) : 0u;
+    const uint32_t l_count = MODE != kWhole && a.list_in ? list_units(__ldcg(&a.in->listed), __ldcg(&a.in->refused)) : 0u;
     const uint32_t l_chunk = max(1u, min(32u, l_count / (gridDim.x * kWarps)));
     uint32_t l_next = 1, l_end = l_count ? 1u : 0u;
     const uint32_t unit_chunks = 1 + tuple_chunks(a.core) + 1;
@@ -168,7 +196,9 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         // ---- this round's work: suffixes once there are 32 pairs; else the
         // deepest depth with 32 candidates; else new roots; else (no more
         // roots) the shallowest depth with any; at last the rest of the pairs
-        const uint32_t full = __ballot_sync(kFull, left >= 32), any = __ballot_sync(kFull, left != 0);
+        // (there is no queue of depth 0: in a whole walk lane 0's `left` counts
+        // rounds, those of suffixes several times)
+        const uint32_t full = __ballot_sync(kFull, left >= 32), any = __ballot_sync(kFull, left != 0) & ~1u;
         uint32_t d = 0;
         bool sfx = spairs >= 32;
         const bool closing = LIM && ++rounds > a.max_rounds;
@@ -176,16 +206,31 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
             if (!spairs) break;
             sfx = true;
         }
+        if (!LIM && lane == 0) left += sfx ? 4 : 1;
         if (!sfx) {
-            if (full) {
+            if (!LIM && (full & 1u)) {
+                // A whole walk's warp looks now and then: once there is nothing
+                // left to take in this pass and most of the chip is idle, what it
+                // has queued goes to the next one, and to all warps.
+                bool end = false;
+                if (lane == 0) {
+                    left = 0;
+                    ++ents;
+                    end = a.look && !(ents & (a.look - 1)) && full > 1 && __ldcg(&a.result->done) >= a.most &&
+                          __ldcg(&a.result->unit) >= a.units &&
+                          (MODE == kWhole || !l_count || __ldcg(&a.in->taken) >= l_count);
+                }
+                if (__any_sync(kFull, end)) break;
+            }
+            if (full > 1) {
                 d = 31 - __clz(full);
             } else {
-                if (LIM && l_end) {  // units that the pass before left come first
+                if (MODE != kWhole && l_end) {  // units that the pass before left come first
                     if (l_next >= l_end) {
                         uint32_t u = 0;
                         if (lane == 0) {
-                            u = __ldcg(&a.result->taken[a.pass - 1]);
-                            if (u < l_count) u = atomicAdd(&a.result->taken[a.pass - 1], l_chunk);
+                            u = __ldcg(&a.in->taken);
+                            if (u < l_count) u = atomicAdd(&a.in->taken, l_chunk);
                         }
                         l_next = __shfl_sync(kFull, u, 0);
                         l_end = min(l_next + l_chunk, l_count);
@@ -203,7 +248,7 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                     // word just to find out took 20 us)
                     unsigned long long u = 0;
                     if (lane == 0) {
-                        if (u_end || (LIM && a.pass)) u = __ldcg(&a.result->unit);
+                        if (u_end || (MODE != kWhole && a.list_in)) u = __ldcg(&a.result->unit);
                         if (u < a.units) u = atomicAdd(&a.result->unit, (unsigned long long)a.chunk);
                     }
                     u_next = __shfl_sync(kFull, u, 0);
@@ -349,6 +394,13 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         }
         __syncwarp();  // queue entries are read by other lanes next
     }
+    // ---- what a pass of a whole walk leaves stays in its queues (k_split)
+    bool open = false;
+    if (!LIM && a.state_out) {
+        if (lane == 0) ents = left = 0;
+        open = __any_sync(kFull, left != 0);
+        if (open && lane == 0) atomicAdd(&a.result->kept, 1u);
+    }
     // ---- what a limited pass leaves: every queue entry as units of kUnit
     // candidates or more (about 64 to an entry at most), whole children or parts of one slice
     if (LIM && __any_sync(kFull, left != 0)) {
@@ -361,15 +413,10 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                 for (uint32_t e = lane; e < n; e += 32) {
                     const Chunk h = q[e];
                     const uint32_t size = max(kUnit, (h.w + 63) / 64);
-                    // children whole in groups (short slices), else one by one in parts
-                    const uint32_t group = max(1u, size / max(h.z, 1u));
                     for (uint32_t at = 0; at < h.w;) {
-                        const uint32_t j = at / h.z, i = at - j * h.z;
-                        Chunk u{h.x + j, h.y + i, min(min(h.z - i, size), h.w - at), 0};
-                        u.w = u.z;
-                        if (i == 0 && u.z == h.z) u.w = h.z * min(group, (h.w - at) / h.z);
+                        const Chunk u = unit_at(h, at, size);
                         at += u.w;
-                        const uint32_t slot = atomicAdd(&a.result->listed[a.pass], 1u);
+                        const uint32_t slot = atomicAdd(&a.out->listed, 1u);
                         if (slot >= kWalkListed) {
                             a.result->gave_up = 1;
                             break;
@@ -404,8 +451,22 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         for (uint32_t w = 0; w < kWarps; ++w) n += cta_sum[w][threadIdx.x];
         if (n) atomicAdd(&a.result->total[blockIdx.x % kWalkTotals][threadIdx.x], n);
     }
+    if (!LIM && a.state_out) {
+        WalkState &st = a.state_out[blockIdx.x * kWarps + warp];
+        if (lane == 0) st.open = open;
+        if (open) {
+            st.ents[lane] = ents;
+            st.left[lane] = left;
+            if (lane == 0) {
+                st.sents = sents;
+                st.spairs = spairs;
+                st.u_next = u_next;
+                st.u_end = u_end;
+            }
+        }
+    }
     // ---- the last CTA to get here hands the call's results to the host
-    if (a.host && a.last) {
+    if (a.last) {
         __shared__ bool mine;
         __threadfence();  // this thread's adds, before its CTA is counted
         __syncthreads();
@@ -414,9 +475,68 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         if (mine) {
             __threadfence();
             const uint4 *const from = reinterpret_cast<const uint4 *>(a.result);
-            for (uint32_t i = threadIdx.x; i < a.host_words; i += kWalkThreads) a.host[i] = __ldcg(from + i);
+            for (uint32_t i = threadIdx.x; a.host && i < a.host_words; i += kWalkThreads) a.host[i] = __ldcg(from + i);
+            if (threadIdx.x == 0) a.result->done = 0;  // for the next pass
         }
     }
+}
+
+// Between two passes of a whole walk: what the warps that closed have queued
+// becomes units for all warps of the next, a warp each, shallowest depths (the
+// largest trees) first, about `share` units a warp and one depth at least.
+// Where the list has no room, the work stays with its warp.
+__global__ void __launch_bounds__(kWalkThreads) k_split(const WalkArgs a) {
+    const uint32_t lane = threadIdx.x & 31u, w = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (w >= a.state_warps || !a.state_in[w].open) return;
+    WalkState &st = a.state_in[w];
+    const uint32_t ents = st.ents[lane], left = st.left[lane], unit_chunks = 1 + tuple_chunks(a.core) + 1;
+    const Chunk *const queues = a.queues + (size_t)w * a.warp_chunks;
+    uint32_t depths = 0, total = 0, mine = 0, at0 = 0;
+    for (uint32_t pass = 0; pass < 2; ++pass) {  // count, then write
+        for (uint32_t d = 1; d < a.core; ++d) {
+            const uint32_t all = __shfl_sync(kFull, left, d), n = within(__shfl_sync(kFull, ents, d), kQueue);
+            if (pass ? !(depths >> d & 1u) : !all || total >= a.share) continue;
+            const Chunk *const q = queues + queue_base(d);
+            const uint32_t size = max(kUnit, (all + a.share - 1) / a.share);
+            for (uint32_t e = lane; e < n; e += 32) {
+                const Chunk h = q[e];
+                for (uint32_t at = 0; at < h.w;) {
+                    const Chunk u = unit_at(h, at, size);
+                    at += u.w;
+                    if (pass) {
+                        Chunk *const o = a.list_out + (size_t)at0++ * unit_chunks;
+                        o[0] = u;
+                        o[1] = Chunk{d, 0, 0, 0};
+                        for (uint32_t x = 0; x * 4 < d; ++x) o[2 + x] = q[(1 + x) * kQueue + e];
+                    } else {
+                        ++mine;
+                    }
+                }
+            }
+            if (!pass) {
+                depths |= 1u << d;
+                total = __reduce_add_sync(kFull, mine);
+            }
+        }
+        if (!pass) {  // room for all of them, or none is listed
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            uint32_t first = 0;
+            if (lane == 0) {
+                first = atomicAdd(&a.out->listed, total);
+                // the first warp without room: the list ends where it would have begun
+                if (first <= kWalkListed && first + total > kWalkListed) a.out->refused = first;
+            }
+            first = __shfl_sync(kFull, first, 0);
+            if (first + total > kWalkListed) return;
+            at0 = first + incl - mine;
+        }
+    }
+    if (depths >> lane & 1u) st.ents[lane] = st.left[lane] = 0;
 }
 
 // Bytes of dynamic shared memory: every lane's tuple.
@@ -449,6 +569,47 @@ inline WalkShape walk_shape(unsigned long long units, uint32_t roots, bool limit
     const uint32_t all = (uint32_t)sms * kCtas;
     return {(uint32_t)chunk,
             (uint32_t)std::max<unsigned long long>(1, std::min<unsigned long long>(all, (need + kWarps - 1) / kWarps))};
+}
+
+inline void (*walk_kernel(const WalkArgs &a, bool lab, WalkMode mode))(const WalkArgs) {
+    if (a.rows && mode == kLater) return lab ? k_walk<true, kLater, true> : k_walk<false, kLater, true>;
+    if (a.rows) return lab ? k_walk<true, kWhole, true> : k_walk<false, kWhole, true>;
+    if (mode == kLater) return lab ? k_walk<true, kLater, false> : k_walk<false, kLater, false>;
+    if (mode == kLimited) return lab ? k_walk<true, kLimited, false> : k_walk<false, kLimited, false>;
+    return lab ? k_walk<true, kWhole, false> : k_walk<false, kWhole, false>;
+}
+
+// The arguments of pass p (see launch_walk); for a whole walk's p > 0 those of
+// the k_split before it as well.
+inline WalkArgs walk_pass(const WalkArgs &args, bool limited, Chunk *lists, int p, uint32_t kept, int sms) {
+    WalkArgs a = args;
+    a.warp_chunks = queue_chunks(a.core);
+    const WalkShape shape = walk_shape(a.units, a.roots, limited, sms);
+    a.chunk = shape.chunk;
+    const uint32_t all = (uint32_t)sms * kCtas;
+    a.ctas = p ? all : shape.ctas;
+    Chunk *const list[2] = {lists, lists + (size_t)kWalkListed * (2 + tuple_chunks(a.core))};
+    a.last = !limited || p + 1 == kWalkPasses;
+    if (limited) {
+        a.max_rounds = kWalkRounds[p];
+        a.list_in = p ? list[(p - 1) & 1] : nullptr;
+        a.list_out = a.last ? nullptr : list[p & 1];
+        a.in = p ? a.result->list + (p - 1) : nullptr;
+        a.out = a.result->list + p;
+    } else if (lists) {
+        // one list (k_split's output, the next pass' input) and the warps' states
+        a.state_out = reinterpret_cast<WalkState *>(list[1]);
+        if (p) {
+            a.list_in = a.list_out = list[0];
+            a.in = a.out = a.result->list;
+            a.state_in = a.state_out;
+            a.state_warps = (p > 1 ? all : shape.ctas) * kWarps;
+            a.share = std::max(64u, kWalkListed / std::max(1u, kept));
+        }
+        a.most = a.ctas - std::min(a.ctas, all / 4);
+        a.look = (p ? kept * 64ull : a.units) < (unsigned long long)all * kWarps ? kWalkLookFew : kWalkLookMany;
+    }
+    return a;
 }
 
 }  // namespace

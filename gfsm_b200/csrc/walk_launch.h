@@ -14,7 +14,16 @@ constexpr int kWalkThreads = 128;
 // pass deals the list to all warps.  What the last one leaves is not walked.
 constexpr int kWalkPasses = 4;
 constexpr uint32_t kWalkRounds[kWalkPasses] = {16, 24, 32, 96};
-constexpr uint32_t kWalkListed = 1u << 18;  // units a list holds
+#ifndef GFSM_WALK_LISTED  // (set by a test that fills a list)
+#define GFSM_WALK_LISTED (1u << 18)
+#endif
+constexpr uint32_t kWalkListed = GFSM_WALK_LISTED;  // units a list holds
+// A whole walk: every so many times 32 rounds a warp looks whether there is
+// work left to take; once there is not, it leaves what it has queued to the
+// next pass, whose warps share it (k_split).  Rounds take 1-2 us (of suffixes
+// up to 8, they count as 4), a pass costs about 25.
+constexpr uint32_t kWalkLookFew = 1;   // fewer units than warps: a warp may hold a whole tree
+constexpr uint32_t kWalkLookMany = 8;
 
 constexpr int kWalkTotals = 32;
 
@@ -22,11 +31,23 @@ struct WalkResult {
     unsigned long long unit;  // units handed out so far
     uint32_t done;     // CTAs of the last pass that have finished
     uint32_t gave_up;  // the last pass left work: the counts are not complete
-    uint32_t listed[kWalkPasses];  // work units each pass left to the next ...
-    uint32_t taken[kWalkPasses];   // ... and how many of them that one has handed out
+    struct List {
+        uint32_t listed, taken;  // work units a pass left to the next, how many of them that one has handed out
+        uint32_t refused;        // (k_split) listed > kWalkListed: where the list ends
+    } list[kWalkPasses];         // limited: one a pass; whole walks use the first
+    uint32_t kept;               // warps of a whole walk's pass that left work
     // candidates, expansions, algorithmic bytes and the bytes of the partial
     // mappings extended (what whole levels would hold), in parts
     unsigned long long total[kWalkTotals][4];
+};
+
+// A warp of a whole walk between two passes: entries and candidates of its
+// queues (lane d: depth d), the suffix queue's entries and pairs, units it has
+// taken and not begun.
+struct WalkState {
+    uint32_t ents[32], left[32];
+    unsigned long long u_next, u_end;
+    uint32_t open, sents, spairs, pad;
 };
 
 struct WalkArgs {
@@ -45,7 +66,7 @@ struct WalkArgs {
     // 6 us in a stream.
     uint4 *host;
     uint32_t host_words;         // in 16 bytes
-    uint32_t last;               // this pass is the call's last (set by launch_walk)
+    uint32_t last;               // this pass may be the call's last (set by walk_pass)
     // mappings of a lone query (null: counts only): up to max_rows rows of k
     // original vertex ids, tuple position i in column col[i]
     uint32_t *rows;
@@ -54,19 +75,28 @@ struct WalkArgs {
     unsigned long long max_rows;
     uint8_t col[MAXQ];
     Chunk *queues;            // walk_queue_bytes(core, sms) of scratch
-    // limited walks only: this pass, its rounds, what the one before left,
-    // where it leaves its own
-    uint32_t pass, max_rounds;
+    // set by walk_pass: a limited pass' rounds, a whole walk's rounds between
+    // looks (in 32; 0: none), and the CTAs that have finished before one hands
+    // its work on; the list that the pass before left
+    // (null: the first), and where this one, or k_split, leaves its own (null:
+    // nowhere); whole walks: the warps' states, those the pass before had, and
+    // the units that k_split makes of one
+    uint32_t max_rounds, look, most;
     const Chunk *list_in;
     Chunk *list_out;
-    uint32_t chunk, warp_chunks;  // set by launch_walk
+    WalkResult::List *in, *out;
+    WalkState *state_in, *state_out;
+    uint32_t state_warps, share;
+    uint32_t chunk, warp_chunks, ctas;
 };
 
 // Bytes of the warps' queues for tuples of up to `core` vertices.
 uint64_t walk_queue_bytes(uint32_t core, int sms);
-// Bytes of the two lists of a limited walk.
+// Bytes of the lists of a call with several passes.
 uint64_t walk_list_bytes(uint32_t core);
-// limited: kWalkPasses passes, with `lists` for what they leave one another.
-cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int sms, cudaStream_t st);
+// Pass p of a call: a limited walk has kWalkPasses, a whole one goes on while
+// warps of its last pass have kept work (`kept`: how many; lists null: one pass).
+cudaError_t launch_walk(const WalkArgs &args, bool lab, bool limited, Chunk *lists, int p, uint32_t kept, int sms,
+                        cudaStream_t st);
 
 }  // namespace gfsm

@@ -88,3 +88,48 @@ def test_limited_walk(monkeypatch, n, m, labels, nq):
         qs.append((q.n, *q.directed(), None, rng.integers(labels // 2, labels, q.n).astype(np.uint32)))
     _counts(ctx, ctx.prepare_queries(qs), data, monkeypatch, None)
     ctx.close()
+
+
+def _path(k, vlabel):
+    q = synth.UGraph(k, np.arange(k - 1, dtype=np.uint32), np.arange(1, k, dtype=np.uint32))
+    q.vlabel = np.array(vlabel, np.uint32)
+    return q
+
+
+@pytest.mark.parametrize("form", ["labels", "edge_labels", "mappings", "clique"])
+def test_few_roots_hand_work_on(monkeypatch, form):
+    """A few warps hold all the work of a walk: ten roots of a rare label, or
+    a clique whose vertices one warp takes at once.  They hand it on to the
+    next pass (a launch each, and one between), with the same counts."""
+    ctx = gfsm_b200.GFSM(device=0, vertex_labels=1)
+    if form == "clique":  # 40 vertices of a 100 x 100 grid
+        g = synth.grid(100, 0.0, 0.0, seed=1)
+        a, b = np.triu_indices(40, 1)
+        g = synth.UGraph(g.n, np.append(g.src, a.astype(np.uint32) * 7), np.append(g.dst, b.astype(np.uint32) * 7))
+        g.vlabel = np.zeros(g.n, np.uint32)
+        q = _path(5, [0] * 5)
+    else:
+        g = synth.er(20000, 16.0 if form == "mappings" else 24.0, seed=3)
+        g.vlabel = np.zeros(g.n, np.uint32)
+        g.vlabel[5::2003] = 1
+        q = _path(5, [0, 1, 0, 0, 0])
+    s, d = g.directed()
+    a, b = q.directed()
+    lab, ql = np.ones(len(s), np.uint32), np.ones(len(a), np.uint32)
+    if form == "edge_labels":
+        lab[:] = 1 + (s ^ d) % 2
+    data = ctx.graph_from_edges(g.n, s, d, lab, g.vlabel).to_device()
+    assert data.info()["max_degree"] <= 64
+    plans = ctx.prepare_queries([(q.n, a, b, ql, q.vlabel)])
+    got, st = ctx.match_count(plans[0], data)
+    assert st["driver"] == 2 and st["launches"] >= 3
+    rows = ctx.match_mappings(plans[0], data, max_rows=1 << 20)[0] if form == "mappings" else None
+    monkeypatch.setenv("GFSM_DRIVER", "host")
+    want, st = ctx.match_count(plans[0], data)
+    assert st["driver"] == 0
+    assert got == want > 0
+    if form == "mappings":  # (every core vertex is enumerated there: far more rounds than the count took)
+        level = ctx.match_mappings(plans[0], data, max_rows=1 << 20)[0]
+        assert len(rows) == want and np.array_equal(rows[np.lexsort(rows.T)], level[np.lexsort(level.T)])
+    plans.close()
+    ctx.close()

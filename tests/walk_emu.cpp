@@ -191,12 +191,14 @@ T *guarded(const std::vector<T> &v) {
 #undef __device__
 #undef __host__
 #undef __forceinline__
+#undef __noinline__
 #undef __launch_bounds__
 #undef __shared__
 #define __global__ static
 #define __device__
 #define __host__
 #define __forceinline__ inline
+#define __noinline__
 #define __launch_bounds__(...)
 #define __shared__ static
 #define GFSM_DYN_SHARED(x) uint32_t *const x = emu::shared
@@ -243,7 +245,7 @@ int main(int argc, char **argv) {
     if (argc < 10) return 2;
     const bool vl = atoi(argv[1]), share = atoi(argv[2]), leaves = atoi(argv[3]), cross = atoi(argv[4]), desc = atoi(argv[5]);
     const std::string form = argv[6];
-    const bool limited = form != "walk";
+    const bool limited = form == "limited" || form == "poison";
     emu::rng.seed((uint64_t)atoll(argv[7]));
     gfsm_limits lim;
     gfsm_limits_default(&lim);
@@ -308,32 +310,42 @@ int main(int argc, char **argv) {
     a.warp_chunks = queue_chunks(w.core);
     const size_t list_chunks = (size_t)kWalkListed * (2 + tuple_chunks(w.core));
     Chunk *const list[2] = {emu::guarded<Chunk>(list_chunks), emu::guarded<Chunk>(list_chunks)};
-    const WalkShape shape = walk_shape(a.units, a.roots, limited, sms);
-    a.chunk = shape.chunk;
+    WalkState *const state = emu::guarded<WalkState>((size_t)sms * kCtas * kWarps);
     const bool labelled = g.elab || g.multi;
-    g_kernel = labelled && limited ? k_walk<true, true, false> : labelled ? k_walk<true, false, false>
-               : limited           ? k_walk<false, true, false> : k_walk<false, false, false>;
     emu::body = [] { g_kernel(g_args); };
-    for (int p = 0; p < (limited ? kWalkPasses : 1); ++p) {
-        a.pass = (uint32_t)p;
-        a.max_rounds = limited ? kWalkRounds[p] : 0;
-        a.list_in = p ? list[(p - 1) & 1] : nullptr;
-        a.list_out = limited && p + 1 < kWalkPasses ? list[p & 1] : nullptr;
-        g_args = a;
-        const uint32_t ctas = p ? (uint32_t)sms * kCtas : shape.ctas;
-        for (uint32_t b = 0; b < ctas; ++b) emu::run_cta(b, ctas);
-        if (form == "poison" && a.list_out)
-            for (uint32_t u = 0; u < std::min(a.result->listed[p], kWalkListed); ++u)
+    WalkResult *r = a.result;
+    uint32_t passes = 0, listed = 0, kept = 0;
+    bool rest = false;
+    for (int p = 0; p < (limited ? kWalkPasses : 1 << 20); ++p) {
+        g_args = walk_pass(a, limited, list[0], p, kept, sms);
+        if (limited) {  // (each list at its own pages)
+            if (g_args.list_in) g_args.list_in = list[(p - 1) & 1];
+            if (g_args.list_out) g_args.list_out = list[p & 1];
+        } else {
+            g_args.state_out = state;
+            if (p) {
+                g_args.state_in = state;
+                *g_args.out = {};
+                r->kept = 0;
+                g_kernel = k_split;
+                const uint32_t ctas = (g_args.state_warps + kWarps - 1) / kWarps;
+                for (uint32_t b = 0; b < ctas; ++b) emu::run_cta(b, ctas);
+                listed += list_units(g_args.out->listed, g_args.out->refused);
+            }
+        }
+        g_kernel = walk_kernel(g_args, labelled, limited ? kLimited : p ? kLater : kWhole);
+        for (uint32_t b = 0; b < g_args.ctas; ++b) emu::run_cta(b, g_args.ctas);
+        if (p) rest = rest || g_args.in->taken < list_units(g_args.in->listed, g_args.in->refused);
+        const uint32_t units = limited && g_args.list_out ? std::min(g_args.out->listed, kWalkListed) : 0;
+        listed += units;
+        passes += units || !passes || !limited;
+        if (form == "poison")
+            for (uint32_t u = 0; u < units; ++u)
                 list[p & 1][(size_t)u * (2 + tuple_chunks(w.core)) + 1].x = 0xfffffff0u + u;
+        kept = r->kept;
+        if (!limited && !kept) break;
     }
-    const WalkResult *r = a.result;
-    bool rest = r->gave_up != 0 || r->unit < a.units;
-    uint32_t passes = 1, listed = 0;
-    for (int p = 0; limited && p + 1 < kWalkPasses; ++p) {
-        rest = rest || r->taken[p] < std::min(r->listed[p], kWalkListed);
-        listed += r->listed[p];
-        passes += r->listed[p] != 0;
-    }
+    rest = rest || r->gave_up != 0 || r->unit < a.units;
     for (int i = 0; i < nq; ++i)
         printf("%llu\n", at[i] < 0 ? 0ull : (unsigned long long)(a.counts[w.slot[at[i]]] * w.mult[at[i]]));
     printf("passes %u listed %u unfinished %d clamped %llu\n", passes, listed, (int)rest, (unsigned long long)g_clamped);
