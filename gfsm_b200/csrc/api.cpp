@@ -45,9 +45,10 @@ Engine *ctx_engine(gfsm_ctx *ctx, const DeviceGraph &g, gfsm_status &rc, std::st
     // MEMLIMIT covers the data graph, the engine's fixed buffers and the arena.
     const uint64_t used = g.bytes + e->small_bytes;
     uint64_t lim_cap = ctx->lim.mem_limit > used ? ctx->lim.mem_limit - used : 0;
-    // what is derived from the graph counts as well, except where a tight
-    // limit would lose much of its arena to it
-    if (lim_cap / 4 > g.aux_bytes) lim_cap -= g.aux_bytes;
+    // What is derived from the graph counts as well.  Its build keeps it to a
+    // quarter of the rest (of a graph built under a larger limit than this
+    // context's, which its owner may use meanwhile, no more is counted).
+    lim_cap -= std::min(g.aux_bytes, lim_cap / 4);
     uint64_t cap = lim_cap;
     // Free device memory is read when the arena is first sized and then every
     // 1024th call (a chance to grow): the query goes through the driver,
@@ -60,12 +61,12 @@ Engine *ctx_engine(gfsm_ctx *ctx, const DeviceGraph &g, gfsm_status &rc, std::st
         avail = avail > (1ull << 30) ? avail - (1ull << 30) : avail / 2;
         cap = std::min(cap, avail);
     }
-    // A large arena is sized in whole steps of 1/16 or less of it, so that the
+    // A large arena is sized in whole steps of 1/64 or less of it, so that the
     // next data graph, a few MB larger, does not free and allocate it again
     // (0.5 s for 22 GB).
     if (!e->arena && cap >= (4ull << 30)) {
-        uint64_t step = 1ull << 28;
-        while (step * 32 <= cap) step *= 2;
+        uint64_t step = 1ull << 25;
+        while (step * 128 <= cap) step *= 2;
         cap -= cap % step;
     }
     // Keep an arena that MEMLIMIT still allows: free-memory readings move a
@@ -89,7 +90,7 @@ gfsm_status ensure_device(gfsm_ctx *ctx, gfsm_graph *g) {
     auto *dg = new (std::nothrow) DeviceGraph();
     if (!dg) return GFSM_ERR_NOMEM;
     std::string err;
-    gfsm_status rc = build_device_graph(g->h, ctx->device, g->vl_mode, *dg, err);
+    gfsm_status rc = build_device_graph(g->h, ctx->device, g->vl_mode, ctx->lim.mem_limit, *dg, err);
     if (rc != GFSM_OK) {
         delete dg;
         return set_err(ctx, rc, "device CCSR build: " + err);
@@ -266,7 +267,7 @@ gfsm_status gfsm_graph_info_get(const gfsm_graph *g, gfsm_graph_info *info) {
         info->multi_edges = d.multi;
         info->n_edge_labels = d.n_edge_labels;
         info->on_device = 1;
-        info->device_bytes = d.bytes;
+        info->device_bytes = d.bytes + d.aux_bytes;
         info->build_alloc_ms = d.build_ms[0];
         info->build_h2d_ms = d.build_ms[1];
         info->build_kernel_ms = d.build_ms[2];

@@ -165,7 +165,7 @@ void free_device_graph(DeviceGraph &g) {
 // with cudaFreeAsync, so the build holds no device-wide synchronisation
 // besides its final stream sync.  Events split the build into allocation,
 // host-to-device copies, device passes and the copies back.
-gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, DeviceGraph &out,
+gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, uint64_t mem_limit, DeviceGraph &out,
                                std::string &err) {
     gfsm_status rc = GFSM_OK;
     const uint32_t n = h.n;
@@ -198,6 +198,8 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     uint32_t groups = 1;
     bool grouped = false;    // rows by label group (rowgrp, nlf)
     uint64_t grp_words = 0;  // rowgrp's words, where it is not rowptr itself
+    uint64_t nlf_bytes = 0, aux_left = 0;
+    bool tables = false;     // rowgrp (beyond rowptr) and nlf are built
     auto t_host0 = std::chrono::steady_clock::now();
 
     {
@@ -284,6 +286,16 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     groups = (uint32_t)out.group_value.size();
     grouped = groups <= DeviceGraph::kMaxRowGroups && n;
     if (grouped && groups > 1) grp_words = (uint64_t)n * groups + 1;
+    if (grouped && groups <= 8) nlf_bytes = n1 * 8;
+    {
+        // The derived tables count towards MEMLIMIT: they may take a quarter
+        // of what it leaves beside the CCSR, and only where that leaves the
+        // search enough to use them (Engine::run's least arena, and a half).
+        const uint64_t ccsr = ((uint64_t)n + 1) * 4 + m * 4 + (one_label ? 0 : m) + (uint64_t)n * 4;
+        const uint64_t rest = mem_limit > ccsr ? mem_limit - ccsr : 0;
+        if (rest >= kWalkMinArena * 3 / 2) aux_left = rest / 4;
+        tables = (grp_words || nlf_bytes) && grp_words * 4 + nlf_bytes <= aux_left;
+    }
 
     // scratch sizes of the CUB passes (queried with null pointers)
     BCHECK(cub::DeviceRadixSort::SortPairs(nullptr, need, (unsigned long long *)nullptr,
@@ -304,18 +316,8 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
     {
         // persistent outputs: rowptr | adj | order | elab
         const uint64_t o_rowptr = 0, o_adj = al((n1 + 1) * 4), o_order = o_adj + al(m1 * 4),
-                       o_elab = o_order + al(n1 * 4), o_grp = o_elab + al(m1), o_nlf = o_grp + al(grp_words * 4),
-                       o_end = o_nlf + (groups <= 8 ? al(n1 * 8) : 0);
-        BCHECK(cudaMalloc(&out.block, o_end));
-        char *b = static_cast<char *>(out.block);
-        out.rowptr = reinterpret_cast<uint32_t *>(b + o_rowptr);
-        out.adj = reinterpret_cast<uint32_t *>(b + o_adj);
-        out.order = reinterpret_cast<uint32_t *>(b + o_order);
-        if (grouped) {
-            out.rowgrp = groups > 1 ? reinterpret_cast<uint32_t *>(b + o_grp) : out.rowptr;
-            if (groups <= 8) out.nlf = reinterpret_cast<uint64_t *>(b + o_nlf);
-        }
-        d_lab2 = reinterpret_cast<uint8_t *>(b + o_elab);  // becomes out.elab when labels differ
+                       o_elab = o_order + al(n1 * 4), o_grp = o_elab + (one_label ? 0 : al(m1)), o_nlf = o_grp + al(grp_words * 4),
+                       o_end = o_nlf + al(nlf_bytes);
         // workspace
         const uint64_t sizes[] = {m1 * 4, m1 * 4, m1, n1 * 4, n1 * 4, n1 * 4, (n1 + 1) * 4, n1 * 4, 64,
                                   n1 * 8, n1 * 8, m1 * 8, m1 * 8, tmp_bytes};
@@ -336,7 +338,27 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
             }
             cudaGetLastError();
         }
-        BCHECK(cudaMallocAsync(reinterpret_cast<void **>(&ws), total, st));
+        // (a device without room for the tables as well does without them)
+        for (;; tables = false) {
+            cudaError_t got = cudaMalloc(&out.block, tables ? o_end : o_grp);
+            if (got != cudaSuccess) out.block = nullptr;
+            else got = cudaMallocAsync(reinterpret_cast<void **>(&ws), total, st);
+            if (got == cudaSuccess) break;
+            ws = nullptr;
+            if (!tables || got != cudaErrorMemoryAllocation) BCHECK(got);
+            cudaGetLastError();
+            if (out.block) cudaFree(out.block);
+            out.block = nullptr;
+            aux_left = 0;
+        }
+        char *b = static_cast<char *>(out.block);
+        out.rowptr = reinterpret_cast<uint32_t *>(b + o_rowptr);
+        out.adj = reinterpret_cast<uint32_t *>(b + o_adj);
+        out.order = reinterpret_cast<uint32_t *>(b + o_order);
+        if (grouped && groups == 1) out.rowgrp = out.rowptr;
+        if (tables && grp_words) out.rowgrp = reinterpret_cast<uint32_t *>(b + o_grp);
+        if (tables && nlf_bytes) out.nlf = reinterpret_cast<uint64_t *>(b + o_nlf);
+        d_lab2 = reinterpret_cast<uint8_t *>(b + o_elab);  // becomes out.elab when labels differ
         char *w = ws;
         auto take = [&](uint64_t bytes) {
             char *r = w;
@@ -395,7 +417,7 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         k_unpack<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.adj, one_label ? nullptr : d_lab2, d_flags);
         k_symmetric<<<grid_for(m, 256), 256, 0, st>>>(d_ekey2, m, bits, out.rowptr, out.adj, d_flags);
     }
-    if (grouped) {
+    if (tables) {
         BCHECK(cudaMemcpyAsync(d_degs, out.group_start.data(), (uint64_t)groups * 4, cudaMemcpyHostToDevice, st));
         k_row_groups<<<grid_for(n, 256), 256, 0, st>>>(out.rowptr, out.adj, n, groups, d_degs, out.rowgrp,
                                                          reinterpret_cast<unsigned long long *>(out.nlf));
@@ -463,15 +485,17 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, Dev
         }
     }
     out.bytes = ((uint64_t)n + 1) * 4 + m * 4 + (out.elab ? m : 0) + (uint64_t)n * 4;
-    out.aux_bytes = grp_words * 4 + (out.nlf ? (uint64_t)n * 8 : 0);
+    out.aux_bytes = tables ? grp_words * 4 + nlf_bytes : 0;
+    aux_left -= std::min(aux_left, out.aux_bytes);
     // Hub adjacency as bits, where rows are long and one edge label makes a
     // check one bit: up to 16,384 vertices (32 MB, held by L2), and no more
     // memory than the CCSR has.
     if (out.n_edge_labels == 1 && !vl_mode && out.max_degree >= kHubRow) {
         uint32_t k = std::min<uint32_t>(kMaxHubs, n) & ~31u;
         while (k > 32 && (uint64_t)k * k / 8 > out.bytes / 2) k = k / 2 & ~31u;
+        while (k > 32 && (uint64_t)k * k / 8 > aux_left) k = k / 2 & ~31u;
         const uint64_t words = (uint64_t)k * k / 32;
-        if (k >= 32 && cudaMalloc(&out.hub_bits, words * 4) == cudaSuccess) {
+        if (k >= 32 && words * 4 <= aux_left && cudaMalloc(&out.hub_bits, words * 4) == cudaSuccess) {
             out.hubs = k;
             out.aux_bytes += words * 4;
             BCHECK(cudaMemsetAsync(out.hub_bits, 0, words * 4, st));

@@ -1112,7 +1112,6 @@ constexpr uint32_t kWalkMaxGroupRow = 1024;
 // Results of up to this many bytes the walk writes to the host itself.
 constexpr uint64_t kWalkHostBytes = 16384;
 constexpr uint64_t kWalkMinLimit = 1ull << 20;
-constexpr uint64_t kWalkMinArena = 256ull << 20;
 
 inline uint64_t div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 

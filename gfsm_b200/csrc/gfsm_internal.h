@@ -80,6 +80,10 @@ void par_ranges(uint64_t n, uint64_t grain, F f) {
 constexpr uint64_t kThreadPays = 1ull << 17;
 constexpr uint64_t kCopyGrain = 1ull << 19;  // items a thread is worth (a copy of 2 MB)
 
+// The least arena for which the walk, and what the derived tables of a data
+// graph serve, is used.
+constexpr uint64_t kWalkMinArena = 256ull << 20;
+
 // ---------------------------------------------------------------------------
 // Host-side graph: the parsed edge lines, labels masked to CCSRRelSize bits.
 // ---------------------------------------------------------------------------
@@ -299,7 +303,8 @@ gfsm_status plan_query(const HostGraph &q, uint32_t rel_bits, Plan &p, const std
 // depths by earlier ones.  Leaves aut = 1 if the search grows too large.
 void plan_symmetry(const HostGraph &q, Plan &p, bool vl);
 // builder.cu
-gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, DeviceGraph &out,
+// mem_limit: the context's, which the derived tables count towards.
+gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, uint64_t mem_limit, DeviceGraph &out,
                                std::string &err);
 void free_device_graph(DeviceGraph &g);
 // engine.cu

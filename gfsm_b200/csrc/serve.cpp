@@ -175,7 +175,8 @@ gfsm_status gfsm_serve_start(gfsm_ctx *ctx, const gfsm_graph *data, const gfsm_s
     if (c.queue_capacity <= 0) c.queue_capacity = 65536;
     s->cfg = c;
     const DeviceGraph &g = *data->dev;
-    const uint64_t avail = ctx->lim.mem_limit > g.bytes ? ctx->lim.mem_limit - g.bytes : 0;
+    uint64_t avail = ctx->lim.mem_limit > g.bytes ? ctx->lim.mem_limit - g.bytes : 0;
+    avail -= std::min(g.aux_bytes, avail / 4);  // as for a call (ctx_engine)
     uint64_t per_slot = avail / (uint64_t)c.slots;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {

@@ -49,7 +49,7 @@ typedef struct {
     uint32_t ccsr_rel_size;    /* CCSRRelSize: edge-label bits kept (1..8), default 8          */
     uint64_t max_soln_size;    /* MAXSOLNSIZE: max partial mappings held per frontier level   */
     uint64_t max_scan_size;    /* MAXSCANSIZE: max candidates examined by one frontier step   */
-    uint64_t mem_limit;        /* MEMLIMIT: device bytes the matcher may hold (graph+frontier) */
+    uint64_t mem_limit;        /* MEMLIMIT: device bytes the matcher may hold (graph, tables derived from it, frontier) */
     uint64_t upper_mem_limit;  /* UPPERMEMLIMIT: cap on any mem_limit override                */
     int32_t  vertex_labels;    /* 0 = reference semantics (labels ignored), 1 = must match    */
     int32_t  degree_filter;    /* 1 = skip candidates whose degree is below the query degree
@@ -72,7 +72,7 @@ typedef struct {
     int32_t  multi_edges;  /* some (u,v) pair appears more than once           */
     int32_t  n_edge_labels;/* distinct edge labels (after CCSRRelSize masking) */
     int32_t  on_device;    /* device CCSR built                                */
-    uint64_t device_bytes;
+    uint64_t device_bytes; /* the device CCSR and the tables derived from it   */
     /* device CCSR build (0 until built): allocation, host-to-device copies,
      * device passes, copies back (CUDA events), and host wall time, ms */
     double   build_alloc_ms, build_h2d_ms, build_kernel_ms, build_d2h_ms, build_wall_ms;
