@@ -171,6 +171,8 @@ gfsm_status build_device_graph(const HostGraph &h, int device, bool vl_mode, uin
     const uint32_t n = h.n;
     const uint64_t m = h.src.size();
     out = DeviceGraph();
+    static std::atomic<uint64_t> serials{0};
+    out.serial = ++serials;
     out.device = device;
     out.n = n;
     out.m = m;

@@ -1536,6 +1536,30 @@ int Engine::pick_variant(const std::vector<const Plan *> &plans, const DeviceGra
     return best;
 }
 
+// Adds what another part of the call (or an attempt at it) took.
+static void add_stats(gfsm_stats &to, const gfsm_stats &from) {
+    to.count += from.count;
+    to.kernel_ms += from.kernel_ms;
+    to.device_ms += from.device_ms;
+    to.steps += from.steps;
+    to.launches += from.launches;
+    to.candidates += from.candidates;
+    to.expansions += from.expansions;
+    to.alg_bytes += from.alg_bytes;
+    to.peak_frontier_bytes = std::max(to.peak_frontier_bytes, from.peak_frontier_bytes);
+    to.h2d_bytes += from.h2d_bytes;
+    to.d2h_bytes += from.d2h_bytes;
+}
+
+// What a limited walk's giving up is remembered by: the data graph, label mode
+// and the work the call's roots bring, beside the workload class.
+static uint64_t skip_class(const std::vector<const Plan *> &plans, const DeviceGraph &g, bool vl, uint64_t entries) {
+    uint64_t h = workload_class(plans, g);
+    for (const uint64_t x : {g.serial, (uint64_t)vl, (uint64_t)(64 - __builtin_clzll(entries | 1))})
+        h = (h ^ x) * 0xff51afd7ed558ccdull, h ^= h >> 32;
+    return h;
+}
+
 // Every later vertex a leaf of the first, with nothing to check but its edge,
 // in label groups that are the same or do not meet: a suffix always holds it.
 inline bool is_star(const DQuery &q) {
@@ -1672,6 +1696,11 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
     bool rest = r->gave_up != 0 || r->unit < a.units;  // work that no pass took on
     for (int p = 0; limited && p + 1 < kWalkPasses; ++p)
         rest = rest || r->list[p].taken < std::min(r->list[p].listed, kWalkListed);
+    // what the attempt cost counts, whether its counts are complete or not
+    st.kernel_ms = st.device_ms = kernel_ms;
+    st.steps = st.launches = (uint32_t)(limited ? passes : 2 * passes - 1);
+    st.h2d_bytes = total;
+    st.d2h_bytes = back;
     if (rest) {
         ran = false;
         return GFSM_OK;
@@ -1687,11 +1716,9 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
             ECHECK(cudaMemcpyAsync(rows_out, a.rows, rows * dq[0].k * 4, cudaMemcpyDeviceToHost, stream));
             ECHECK(cudaStreamSynchronize(stream));
         }
-        st.d2h_bytes = rows * dq[0].k * 4;
+        st.d2h_bytes += rows * dq[0].k * 4;
         if (n_rows) *n_rows = rows;
     }
-    st.kernel_ms = st.device_ms = kernel_ms;
-    st.steps = st.launches = (uint32_t)(limited ? passes : 2 * passes - 1);
     for (const auto &t : r->total) {
         st.candidates += t[0];
         st.expansions += t[1];
@@ -1699,8 +1726,6 @@ gfsm_status Engine::run_walk(const std::vector<const Plan *> &plans, const std::
         st.peak_frontier_bytes += t[3];
     }
     st.peak_frontier_bytes = std::min<uint64_t>(st.peak_frontier_bytes, arena_cap);
-    st.h2d_bytes = total;
-    st.d2h_bytes += back;
     st.driver = 2;
     return GFSM_OK;
 }
@@ -1889,17 +1914,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
                 gfsm_stats r{};
                 rc = run(rest, g, lim, counts.data(), &r, nullptr, 0, nullptr, err, variant, part, nparts);
                 for (size_t i = 0; i < rest.size(); ++i) counts_out[others[i]] = counts[i];
-                r.count += st.count;
-                r.kernel_ms += st.kernel_ms;
-                r.device_ms += st.device_ms;
-                r.steps += st.steps;
-                r.launches += st.launches;
-                r.candidates += st.candidates;
-                r.expansions += st.expansions;
-                r.alg_bytes += st.alg_bytes;
-                r.peak_frontier_bytes = std::max(r.peak_frontier_bytes, st.peak_frontier_bytes);
-                r.h2d_bytes += st.h2d_bytes;
-                r.d2h_bytes += st.d2h_bytes;
+                add_stats(r, st);
                 st = r;
             }
             st.wall_ms =
@@ -1920,7 +1935,8 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
             for (uint32_t i = 0; i < na && entries <= kGraphRootEntries; ++i)
                 entries += (uint64_t)g.h_rowptr[rhi[i]] - g.h_rowptr[rlo[i]];
             if (entries <= kGraphRootEntries) {
-                Skip &skip = walk_skip[workload_class(plans, g)];
+                if (walk_skip.size() >= 4096) walk_skip.clear();
+                Skip &skip = walk_skip[skip_class(plans, g, vl_on, entries)];
                 if (skip.left) {
                     --skip.left;
                 } else {
@@ -1941,8 +1957,13 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
             if (stats) *stats = st;
             return rc;
         }
-        return run(plans, g, lim, counts_out, stats, rows_out, max_rows, n_rows, err,
-                   plans.size() <= 1 ? 0 : pick_variant(plans, g, lim, err), part, nparts);
+        gfsm_stats level{};
+        rc = run(plans, g, lim, counts_out, &level, rows_out, max_rows, n_rows, err,
+                 plans.size() <= 1 ? 0 : pick_variant(plans, g, lim, err), part, nparts);
+        add_stats(level, st);
+        level.wall_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
+        if (stats) *stats = level;
+        return rc;
     }
     const uint64_t fan_cap = 0xffffffffull / (row_max * kWarpStage);
     std::vector<uint32_t> root_rep, fan_list, final_rep(na);

@@ -34,7 +34,7 @@ struct Engine {
     int sm_count = 0;
     WalkTables walk_tables;        // the walk's tables and a call's device plans, reused by the next call
     std::vector<DQuery> dq_kept;
-    // walks on long-row data that gave up, per workload class: how many calls
+    // walks on long-row data that gave up, per data graph and work: how many calls
     // to leave to the level steps before the next try, and how many after that
     struct Skip {
         uint32_t left = 0, next = 8;

@@ -118,6 +118,7 @@ struct DeviceGraph {
     // in degree order, a skewed graph, else null
     uint32_t *hub_bits = nullptr;
     uint32_t hubs = 0;
+    uint64_t serial = 0;              // tells the process' data graphs apart
     void *block = nullptr;            // the one allocation rowptr, adj, order and elab live in
     bool symmetric = false, multi = false;
     int n_edge_labels = 0;
