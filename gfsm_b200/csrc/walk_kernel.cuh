@@ -98,6 +98,12 @@ __device__ __forceinline__ void deal(uint32_t n, uint32_t lane, uint32_t &incl, 
     local = lane - __shfl_sync(kFull, excl, from);
 }
 
+// Bits of a lane's total from which it is added to the call's.
+#ifndef GFSM_SPILL_BITS  // (set by a test)
+#define GFSM_SPILL_BITS 30
+#endif
+constexpr uint32_t kSpillBits = GFSM_SPILL_BITS;
+
 // Candidates in a unit that a limited pass leaves, at least: few, since the
 // search below each can be long and there are far more warps than units.
 constexpr uint32_t kUnit = 8;
@@ -192,6 +198,18 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
         fslot = slot;
         fcount += n;
     };
+    // A lane's totals have 32 bits: they are added to the call's before they
+    // can wrap (a round adds under 2^27 to each, several rounds 2^30 at most).
+    auto spill = [&] {
+        if (__any_sync(kFull, (bytes | front) >> kSpillBits)) {
+            unsigned long long *const to = a.result->total[blockIdx.x % kWalkTotals];
+            atomicAdd(to, (unsigned long long)cand);
+            atomicAdd(to + 1, (unsigned long long)kept);
+            atomicAdd(to + 2, (unsigned long long)bytes);
+            atomicAdd(to + 3, (unsigned long long)front);
+            cand = kept = bytes = front = 0;
+        }
+    };
     for (;;) {
         // ---- this round's work: suffixes once there are 32 pairs; else the
         // deepest depth with 32 candidates; else new roots; else (no more
@@ -212,6 +230,7 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                 // A whole walk's warp looks now and then: once there is nothing
                 // left to take in this pass and most of the chip is idle, what it
                 // has queued goes to the next one, and to all warps.
+                spill();
                 bool end = false;
                 if (lane == 0) {
                     left = 0;
@@ -298,10 +317,8 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                     const uint32_t nleaf = __ldg(&sx->nleaf);
                     if (nleaf > 1 && first) front += (uint32_t)tuple_bytes(nc - 1);
                     if (nleaf > 2) front += first * (uint32_t)tuple_bytes(nc);
-                    // a hub's row is added for each of its suffixes, under 2^29 at a time
-                    bytes = min(bytes, 1u << 31);
-                    front = min(front, 1u << 31);
                 }
+                spill();  // (a hub's row is added for each of its suffixes)
                 __syncwarp();
                 continue;
             }

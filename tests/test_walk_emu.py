@@ -36,6 +36,12 @@ def exe_short_list(tmp_path_factory):
     return _build(tmp_path_factory, "-DGFSM_WALK_LISTED=40")
 
 
+@pytest.fixture(scope="module")
+def exe_spill(tmp_path_factory):
+    """A lane's totals are added to the call's from 64 on."""
+    return _build(tmp_path_factory, "-DGFSM_SPILL_BITS=6")
+
+
 def _few_roots():
     """Five vertices of label 1, the rest label 0, rows of about 16; a path
     whose search starts at its one vertex of label 1."""
@@ -125,3 +131,15 @@ def test_a_full_list(exe_short_list, tmp_path):
     assert got == want and st["unfinished"] == 0 and st["clamped"] == 0
     _, st = _run(exe_short_list, tmp_path, paths, "limited", 1)
     assert st["unfinished"] == 1 and st["clamped"] == 0
+
+
+@pytest.mark.parametrize("case", ["grid", "few_roots", "ba"])
+def test_totals_in_parts(exe, exe_spill, tmp_path, case):
+    """A call's totals are the same however often a lane's are added to them."""
+    make, *rest = CASES[case]
+    paths, want = _case(tmp_path, make(), *rest)
+    got, st = _run(exe, tmp_path, paths, "walk", 1)
+    parts, sp = _run(exe_spill, tmp_path, paths, "walk", 1)
+    assert got == parts == want
+    for k in ("candidates", "kept", "bytes", "front"):
+        assert st[k] == sp[k] > 0

@@ -7,7 +7,8 @@
 //   walk_emu <vertex labels> <share> <leaves> <cross> <desc> <form> <seed> <data> <query>...
 // form: walk, limited, or poison (limited, with a depth out of range in every
 // list unit).  Prints each query's count (one line each), then
-// "passes <p> listed <l> unfinished <0|1> clamped <c>".
+// "passes <p> listed <l> unfinished <0|1> clamped <c> candidates <n> kept <n>
+// bytes <n> front <n>".
 #include <setjmp.h>
 #include <sys/mman.h>
 #include <ucontext.h>
@@ -348,6 +349,10 @@ int main(int argc, char **argv) {
     rest = rest || r->gave_up != 0 || r->unit < a.units;
     for (int i = 0; i < nq; ++i)
         printf("%llu\n", at[i] < 0 ? 0ull : (unsigned long long)(a.counts[w.slot[at[i]]] * w.mult[at[i]]));
-    printf("passes %u listed %u unfinished %d clamped %llu\n", passes, listed, (int)rest, (unsigned long long)g_clamped);
+    unsigned long long total[4] = {};
+    for (const auto &t : r->total)
+        for (int i = 0; i < 4; ++i) total[i] += t[i];
+    printf("passes %u listed %u unfinished %d clamped %llu candidates %llu kept %llu bytes %llu front %llu\n", passes, listed,
+           (int)rest, (unsigned long long)g_clamped, total[0], total[1], total[2], total[3]);
     return 0;
 }
