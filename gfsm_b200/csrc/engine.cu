@@ -1755,7 +1755,7 @@ gfsm_status Engine::run(const std::vector<const Plan *> &plans, const DeviceGrap
     const bool force_host = trace || (env_drv && strcmp(drv, "graph")) || (!env_drv && tune_driver == 0);
     // The walk (walk.cu) takes counting calls, and a lone query's mappings,
     // on data of short rows: no level is written, and a lane's row scans are
-    // short (one grid query 294 -> 96 us, 4,096 of them 103 -> 62 ms).  A call
+    // short (one grid query 294 -> 84-102 us, 4,096 of them 103 -> 55 ms).  A call
     // that names a level-step setting, caps its candidates or bounds its
     // levels tightly gets the level steps, whose schedule those settings
     // describe.

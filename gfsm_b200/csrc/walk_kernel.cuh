@@ -12,13 +12,21 @@
 // their neighbours' labels.
 //
 // Bound: instruction issue and the latency of a round's dependent loads
-// (queue entry, row entry, row pointers by label group);
-// ncu on 64 grid queries: 60-70% issue active, DRAM 1.1 TB/s.  Before (level
-// steps) and after, whole calls: one 5-vertex query on 2,000 vertices 208 ->
-// 42 us, one 7-vertex query on the 1,400 x 1,400 grid 294 -> 96 us, 64 such
-// queries of 4-10 vertices 3.4 -> 1.4 ms, 4,096 of them from edge lists 102
-// -> 62 ms (kernel 57 ms).  One lane per search (no queues) left 9 of 32
-// lanes active: 4,096 queries took 507 ms.
+// (queue entry, row entry, row pointers by label group); ncu on
+// 64 grid queries, cold caches: 48% issue active with 22 of 32 lanes, 8.7
+// long-scoreboard stalls an issue, DRAM 0.62 TB/s.
+// Before (level steps) and after, whole calls: one 5-vertex query on 2,000
+// vertices 208 -> 40 us, one 7-vertex query on the 1,400 x 1,400 grid 294 ->
+// 84-102 us, 64 such queries of 4-10 vertices 3.4 -> 1.36-1.46 ms, 4,096 of
+// them from edge lists 102 -> 55 ms.  One lane per search (no queues) left 9
+// of 32 lanes active: 4,096 queries took 507 ms.
+//
+// Work is shared by passes.  A warp keeps the trees below its roots, and most
+// calls end so.  Where a few warps hold most of the work, they stop, k_split
+// cuts their queues into units, and all warps of the next pass take those: ten
+// roots on rows of 30, a path of six vertices, 24.5 -> 0.95 ms; a clique of 48
+// in a grid, a path of five, 9.1 -> 1.9 ms.  (The level steps take 0.5 and 0.3
+// ms there: their tiles split any row evenly.)  No warp waits for another.
 //
 // Compiled by the host compiler too, with 32-lane stand-ins for the warp
 // intrinsics (the test that runs every lane of it in a random order).
@@ -36,8 +44,8 @@ namespace {
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kWarps = kWalkThreads / 32;
 // CTAs an SM runs: 32 warps at 64 registers.  40 warps (48 registers) hide
-// more latency but cost instructions: 4,096 grid queries 57.4 against 58.4
-// ms, but one 67 against 63 us, 32 edge-labelled queries 215 against 197 us.
+// more latency but cost instructions (before the loops were rolled, walk.cuh):
+// 4,096 grid queries 57.4 against 58.4 ms, but one 67 against 63 us, 32 edge-labelled queries 215 against 197 us.
 constexpr uint32_t kCtas = 8;
 
 // A word read back from a queue or a list is clamped to the array it indexes
@@ -263,8 +271,8 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
                 }
                 if (more && u_next >= u_end) {
                     // (a warp's first take goes straight to the counter; later it
-                    // looks whether any are left: 5,920 warps adding to one
-                    // word just to find out took 20 us)
+                    // looks whether any are left: all warps adding to one
+                    // word just to find out took 20 us, with 40 warps an SM)
                     unsigned long long u = 0;
                     if (lane == 0) {
                         if (u_end || (MODE != kWhole && a.list_in)) u = __ldcg(&a.result->unit);
@@ -447,8 +455,8 @@ __global__ void __launch_bounds__(kWalkThreads, kCtas) k_walk(const WalkArgs a) 
             }
         }
     }
-    // ---- counts and totals.  5,920 warps adding to the same words one by one
-    // took 25 us: a warp whose lanes hold one slot's count adds once, a CTA its
+    // ---- counts and totals.  All warps adding to the same words one by one
+    // took 25 us (with 40 warps an SM): a warp whose lanes hold one slot's count adds once, a CTA its
     // totals once, to one of kWalkTotals places.
     const uint32_t hold = __ballot_sync(kFull, fcount != 0);
     if (hold) {

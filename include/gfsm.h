@@ -97,7 +97,8 @@ typedef struct {
     uint64_t d2h_bytes;          /* device->host bytes copied by the call          */
     int32_t  tile_variant;       /* tile geometry the autotuner chose (0..3)        */
     uint32_t launches;           /* kernels the call launched (graph nodes included) */
-    int32_t  driver;             /* 2: the whole search ran as one kernel (the walk);
+    int32_t  driver;             /* 2: the whole search ran as the walk (one kernel,
+                                    or a few passes of it);
                                     1: the level steps as one CUDA graph launch;
                                     0: the level steps driven by the host          */
     int32_t  graph_error;        /* a graph was wanted but could not be built (cudaError_t) */
